@@ -86,12 +86,16 @@ agg_layout_k(AggBatch b, uint64_t* scratch, uint64_t scratch_stride)
     const uint64_t v = p < L.positions ? s[p] : 0;
     uint64_t tile_total;
     const uint64_t ex = block_exclusive_scan(v, warp_tot, tile_total);
-    if (p < L.positions)
+    if (p < L.positions) {
       L.offsets[p] = carry + ex;
+      L.host_offsets[p] = carry + ex;
+    }
     carry += tile_total;
   }
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0) {
     L.offsets[L.positions] = carry;
+    L.host_offsets[L.positions] = carry;
+  }
   // the padding that rounds each shard group up to the alignment is written
   // as zeros (no stale buffer bytes reach the shard files), and so is the
   // alignment's worth of bytes after the batch: a delivery write of a run
@@ -174,7 +178,7 @@ __global__ void __launch_bounds__(256) tail_copy_k(TailCopies t)
 // ---- shard index and crc32c ------------------------------------------------
 
 constexpr uint32_t kCrcPoly = 0x82F63B78u; // Castagnoli, reflected
-constexpr int kIndexThreads = 128;
+constexpr int kIndexThreads = 256;
 
 // a * b mod P in the reflected representation (bit 31 = x^0); `a` is a
 // power of x (never 0).  The combination of segment CRCs through
@@ -191,73 +195,137 @@ __device__ uint32_t crc_mulmod(uint32_t a, uint32_t b)
   return p;
 }
 
-// x^(8 n) mod P
-__device__ uint32_t crc_xpow8(uint64_t n)
+// x^(8 * 2^k) mod P for k = 0 .. 47, each the square of the one before.
+struct CrcPowers
 {
-  uint32_t p = 0x80000000u, base = 0x00800000u; // x^0, x^8
-  while (n) {
-    if (n & 1)
-      p = crc_mulmod(p, base);
-    base = crc_mulmod(base, base);
-    n >>= 1;
+  uint32_t p[48];
+};
+constexpr uint32_t crc_mulmod_host(uint32_t a, uint32_t b)
+{
+  uint32_t p = 0;
+  for (int i = 0; i < 32; ++i) {
+    if (a & (0x80000000u >> i))
+      p ^= b;
+    b = (b & 1) ? (b >> 1) ^ kCrcPoly : b >> 1;
   }
   return p;
 }
+constexpr CrcPowers crc_powers()
+{
+  CrcPowers t{};
+  t.p[0] = 0x00800000u; // x^8
+  for (int k = 1; k < 48; ++k)
+    t.p[k] = crc_mulmod_host(t.p[k - 1], t.p[k - 1]);
+  return t;
+}
+__constant__ CrcPowers kCrcPowers = crc_powers();
+
+// x^(8 n) mod P: one multiplication per set bit of n
+__device__ uint32_t crc_xpow8(uint64_t n)
+{
+  uint32_t p = 0x80000000u; // x^0
+  for (int k = 0; n && k < 48; ++k, n >>= 1)
+    if (n & 1)
+      p = crc_mulmod(p, kCrcPowers.p[k]);
+  return p;
+}
+
+// Working memory of one CTA's index checksum.
+struct CrcShared
+{
+  uint32_t table[256];
+  uint32_t warp[kIndexThreads / 32];
+  uint32_t mul[8];   // x^(64 per 2^k): joins 2^k threads' segments to the next
+  uint32_t init;     // ~0 carried over the whole index
+  uint32_t crc;
+};
+
+// The parts of the checksum that depend on the index's length only, so
+// that they are computed while the entries' loads are in flight.
+__device__ void index_crc_prepare(CrcShared& S, uint64_t nwords)
+{
+  const unsigned tid = threadIdx.x;
+  const uint64_t per = (nwords + kIndexThreads - 1) / kIndexThreads;
+  for (unsigned i = tid; i < 256; i += kIndexThreads) {
+    uint32_t c = i;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      c = (c & 1) ? (c >> 1) ^ kCrcPoly : c >> 1;
+    S.table[i] = c;
+  }
+  if (tid < 8)
+    S.mul[tid] = crc_xpow8((per * 8) << tid);
+  else if (tid == 32) // another warp's lane: side by side with the above
+    S.init = crc_mulmod(crc_xpow8(nwords * 8), 0xFFFFFFFFu);
+}
 
 // crc32c of the index words idx[0 .. nwords) (u64, little endian), by the
-// whole CTA: one segment per thread, combined by thread 0.
-__device__ uint32_t index_crc32c(const uint64_t* idx, uint64_t nwords, uint32_t* table,
-                                 uint32_t* part)
+// whole CTA (crc_prepare before it, with a barrier in between).  A CRC that
+// starts from 0 ignores leading zeros, so the words are taken as if padded
+// in front to a segment of `per` words for every thread: all segments then
+// have one length, and neighbours are joined pairwise (left * x^len + right)
+// in log2(threads) steps with one multiplier each; the starting value ~0 is
+// added at the end.
+__device__ void index_crc32c(CrcShared& S, const uint64_t* idx, uint64_t nwords)
 {
-  const unsigned tid = threadIdx.x, nt = blockDim.x;
-  const uint64_t per = (nwords + nt - 1) / nt; // words per thread
-  const uint64_t w0 = (tid * per < nwords ? tid * per : nwords), w1 = (w0 + per < nwords ? w0 + per : nwords);
+  constexpr unsigned kAll = 0xffffffffu;
+  const unsigned tid = threadIdx.x, lane = tid & 31;
+  const uint64_t per = (nwords + kIndexThreads - 1) / kIndexThreads;
+  const uint64_t padded = per * kIndexThreads - nwords;
+  const uint64_t e = (tid + 1) * per; // past the segment's end, padded
   uint32_t c = 0;
-  for (uint64_t w = w0; w < w1; ++w) {
-    uint64_t v = idx[w];
-    for (int k = 0; k < 8; ++k) {
-      c = table[(c ^ uint32_t(v)) & 0xFF] ^ (c >> 8);
-      v >>= 8;
+  if (e > padded) {
+    const uint64_t w1 = e - padded, w0 = w1 > per ? w1 - per : 0;
+#pragma unroll 4
+    for (uint64_t w = w0; w < w1; ++w) {
+      uint64_t v = idx[w];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        c = S.table[(c ^ uint32_t(v)) & 0xFF] ^ (c >> 8);
+        v >>= 8;
+      }
     }
   }
-  part[tid] = c;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const uint32_t r = __shfl_down_sync(kAll, c, 1u << k);
+    if ((lane & ((2u << k) - 1)) == 0)
+      c = crc_mulmod(S.mul[k], c) ^ r;
+  }
+  if (lane == 0)
+    S.warp[tid >> 5] = c;
   __syncthreads();
-  uint32_t crc = 0;
-  if (tid == 0) {
-    uint32_t st = 0xFFFFFFFFu;
-    const uint32_t xfull = crc_xpow8(per * 8);
-    for (unsigned t = 0; t < nt; ++t) {
-      const uint64_t a = t * per < nwords ? t * per : nwords;
-      const uint64_t b = a + per < nwords ? a + per : nwords;
-      if (b <= a)
-        break;
-      const uint32_t x = (b - a == per) ? xfull : crc_xpow8((b - a) * 8);
-      st = crc_mulmod(x, st) ^ part[t];
+  if (tid < 32) {
+    static_assert(kIndexThreads == 256, "three steps join the warps");
+    c = lane < kIndexThreads / 32 ? S.warp[lane] : 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const uint32_t r = __shfl_down_sync(kAll, c, 1u << k);
+      if ((lane & ((2u << k) - 1)) == 0)
+        c = crc_mulmod(S.mul[5 + k], c) ^ r;
     }
-    crc = st ^ 0xFFFFFFFFu;
+    if (lane == 0)
+      S.crc = c ^ S.init ^ 0xFFFFFFFFu;
   }
   __syncthreads();
-  return crc;
 }
 
 // A CTA per (level, shard) (shards beyond the grid's y extent looped): the
 // level's runs in order (each shard's cursor depends on the runs before),
-// the entries of a run in parallel.
+// the entries of a run in parallel.  Bound by latency: a few dependent
+// loads, then the checksum's chains.  What it spent its time on was one
+// thread joining 128 segment CRCs (a 32-step multiplication each) and reads
+// of offsets and sizes in mapped host memory; both are gone (pairwise joins,
+// device copies).  A stream pass that ends two batches went from 694 to
+// 600 us (120-chunk shards) and from 480 to 356 us (1092-chunk shards).
 __global__ void __launch_bounds__(kIndexThreads) index_k(IndexBatch b)
 {
-  __shared__ uint32_t table[256];
-  __shared__ uint32_t part[kIndexThreads];
-  __shared__ uint32_t crc_sh;
+  __shared__ CrcShared C;
   const IndexLevel& L = b.lv[blockIdx.x];
   const unsigned tid = threadIdx.x, nt = blockDim.x;
   if (blockIdx.y >= L.shards)
     return;
-  for (unsigned i = tid; i < 256; i += nt) {
-    uint32_t c = i;
-    for (int k = 0; k < 8; ++k)
-      c = (c & 1) ? (c >> 1) ^ kCrcPoly : c >> 1;
-    table[i] = c;
-  }
+  index_crc_prepare(C, L.cps_total * 2);
   __syncthreads();
   const uint64_t sa = b.alignment;
   const uint64_t nidx = L.cps_total * 16, total = nidx + 4;
@@ -269,10 +337,7 @@ __global__ void __launch_bounds__(kIndexThreads) index_k(IndexBatch b)
     uint32_t nfinal = 0;
     // the shard's final index blob: padding, index, crc32c; then reset
     auto finalize = [&](uint8_t* blob) {
-      const uint32_t crc = index_crc32c(idx, L.cps_total * 2, table, part);
-      if (tid == 0)
-        crc_sh = crc;
-      __syncthreads();
+      index_crc32c(C, idx, L.cps_total * 2);
       for (uint64_t i = tid; i < pad; i += nt)
         blob[i] = 0;
       if ((pad & 3) == 0) {
@@ -286,7 +351,7 @@ __global__ void __launch_bounds__(kIndexThreads) index_k(IndexBatch b)
           blob[pad + i] = src[i];
       }
       if (tid < 4)
-        blob[pad + nidx + tid] = uint8_t(crc_sh >> (8 * tid));
+        blob[pad + nidx + tid] = uint8_t(C.crc >> (8 * tid));
       __syncthreads();
       for (uint64_t i = tid; i < L.cps_total * 2; i += nt)
         idx[i] = ~uint64_t(0);
@@ -297,7 +362,7 @@ __global__ void __launch_bounds__(kIndexThreads) index_k(IndexBatch b)
       cur = 0;
     } else {
       for (uint32_t r = 0; r < L.n_runs; ++r) {
-        const IndexRun R = L.runs[r];
+        const IndexRun R = r ? L.runs[r] : L.run0;
         const uint64_t j0 = s * L.n_active * cpi + uint64_t(R.a0) * cpi;
         const uint64_t j1 = j0 + uint64_t(R.run) * cpi;
         const uint64_t base = L.offsets[j0];

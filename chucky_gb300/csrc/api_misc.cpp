@@ -374,9 +374,10 @@ int estimate_stream(const tile_stream_configuration* config,
     const uint64_t pos = cap * V.covering;
     const uint64_t sa = config->shard_alignment;
     const uint64_t nsh = V.covering / V.cps_inner;
-    agg_host += 2 * ((pos + 1) * 8 + pos * 8 + 8 + cap * M * P.max_out +
+    agg_host += 2 * ((pos + 1) * 8 + cap * M * P.max_out +
                      (sa ? (nsh + 1) * sa : 0) + 64);
-    agg_dev += 4 * cap * M * 4 + (pos + 1) * 8;
+    // shard-order tables, scan scratch, both slots' offsets and sizes
+    agg_dev += 4 * cap * M * 4 + (pos + 1) * 8 + 2 * ((pos + 1) * 8 + pos * 8 + 8);
     if (config->codec.id != CODEC_NONE) // device copy of both delivery slots
       agg_dev += 2 * (cap * M * P.max_out + (sa ? (nsh + 1) * sa : 0) + 64);
     shard += V.shard_inner_count * V.cps_total * 16;

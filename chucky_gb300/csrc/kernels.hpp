@@ -117,8 +117,9 @@ struct AggLevel
   uint64_t n;              // number of mapped chunks
   uint64_t positions;      // n_active * covering
   uint64_t group;          // n_active * cps_inner (page-pad unit)
-  uint64_t* offsets;       // [positions + 1] (written)
-  uint64_t* real_sizes;    // [positions] pre-padding sizes (written)
+  uint64_t* offsets;       // [positions + 1] (written; device)
+  uint64_t* host_offsets;  // the same for the host (mapped)
+  uint64_t* real_sizes;    // [positions] pre-padding sizes (written; device)
   uint8_t* out;            // shard-ordered bytes (written)
 };
 
@@ -157,7 +158,8 @@ struct IndexLevel
   uint64_t* cursor;            // [shards] bytes in each shard file so far
   const uint64_t* offsets;     // the batch's shard-order offsets (or null)
   const uint64_t* real_sizes;  // pre-padding sizes
-  const IndexRun* runs;        // [n_runs]
+  IndexRun run0;               // runs[0], by value
+  const IndexRun* runs;        // [n_runs] (mapped)
   uint32_t n_runs;
   uint32_t n_active;           // active epochs of the level in the batch
   uint64_t cpi;                // chunks per shard per epoch (inner)

@@ -455,7 +455,8 @@ int Stream::setup_aggregate()
       D.positions_cap = positions;
       D.data_cap = data;
       CK(cudaHostAlloc(&D.offsets, (positions + 1) * 8, cudaHostAllocMapped));
-      CK(cudaHostAlloc(&D.real_sizes, positions * 8 + 8, cudaHostAllocMapped));
+      CK(cudaMalloc(&D.d_offsets, (positions + 1) * 8));
+      CK(cudaMalloc(&D.real_sizes, positions * 8 + 8));
       CK(cudaHostAlloc(&D.data, data, cudaHostAllocMapped));
       // compressed batches are gathered in device memory and copied to the
       // host by the copy engine (faster than SM stores over the link)
@@ -525,7 +526,8 @@ void Stream::release()
       cudaFreeHost(slot[i].lv[l].runs);
       cudaFreeHost(slot[i].lv[l].blobs);
       cudaFreeHost(slot[i].lv[l].offsets);
-      cudaFreeHost(slot[i].lv[l].real_sizes);
+      cudaFree(slot[i].lv[l].d_offsets);
+      cudaFree(slot[i].lv[l].real_sizes);
       cudaFreeHost(slot[i].lv[l].data);
       cudaFree(slot[i].lv[l].d_data);
     }
@@ -862,7 +864,8 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
     A.positions = uint64_t(na) * V.covering;
     A.group = uint64_t(na) * V.cps_inner;
     DeliverySlot::Level& D = S.lv[l];
-    A.offsets = D.offsets;
+    A.offsets = D.d_offsets;
+    A.host_offsets = D.offsets;
     A.real_sizes = D.real_sizes;
     A.out = D.d_data ? D.d_data : D.data;
     D.positions = A.positions;
@@ -917,9 +920,10 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
       IndexLevel& X = ib.lv[ib.nlevels++];
       X.index = d_index[l];
       X.cursor = d_cursor[l];
-      X.offsets = D.offsets;
+      X.offsets = D.d_offsets;
       X.real_sizes = D.real_sizes;
       X.runs = D.runs;
+      X.run0 = D.runs[0];
       X.n_runs = D.n_runs;
       X.n_active = S.active[l];
       X.cpi = V.cps_inner;
@@ -947,7 +951,7 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
       TailCopy& t = tails.lv[tails.n++];
       t.dst = D.data;
       t.src = D.d_data;
-      t.total = D.offsets + D.positions; // mapped: written by the aggregation
+      t.total = D.d_offsets + D.positions; // written by the aggregation
       t.extra = cfg.shard_alignment;     // the zeroed slack after the batch
       t.start = D.copied;
       tail_max = std::max(tail_max, D.data_cap - D.copied);

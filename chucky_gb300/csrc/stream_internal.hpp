@@ -30,8 +30,11 @@ struct DeliverySlot
 {
   struct Level
   {
-    uint64_t* offsets = nullptr;    // [positions + 1]
-    uint64_t* real_sizes = nullptr; // [positions]
+    uint64_t* offsets = nullptr;    // [positions + 1] (mapped, for the host)
+    // the kernels' own copies: they read the offsets for every chunk, and a
+    // read of mapped memory crosses the link
+    uint64_t* d_offsets = nullptr;  // [positions + 1]
+    uint64_t* real_sizes = nullptr; // [positions], pre-padding
     uint8_t* data = nullptr;        // host (mapped) shard-ordered bytes
     uint8_t* d_data = nullptr;      // device copy (compressed codecs)
     uint64_t positions_cap = 0, data_cap = 0;
