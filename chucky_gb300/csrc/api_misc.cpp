@@ -378,7 +378,7 @@ int estimate_stream(const tile_stream_configuration* config,
                      (sa ? (nsh + 1) * sa : 0) + 64);
     // shard-order tables, scan scratch, both slots' offsets and sizes
     agg_dev += 4 * cap * M * 4 + (pos + 1) * 8 + 2 * ((pos + 1) * 8 + pos * 8 + 8);
-    if (config->codec.id != CODEC_NONE) // device copy of both delivery slots
+    if (chucky::delivery_through_device(*config, P)) // device copy of both slots
       agg_dev += 2 * (cap * M * P.max_out + (sa ? (nsh + 1) * sa : 0) + 64);
     shard += V.shard_inner_count * V.cps_total * 16;
   }

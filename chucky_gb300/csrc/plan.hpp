@@ -94,6 +94,21 @@ uint64_t ravel(int rank,
                const int64_t* strides,
                uint64_t idx);
 
+// Whether a batch's shard-ordered bytes are gathered in device memory and
+// moved to the host by the copy engine, rather than stored by the gather
+// kernel into mapped host memory.
+//
+// The copy engine moves 190 GB/s over the link, SM stores 94 GB/s, and the
+// next batch's kernels run beside the copy; but the copy is one more step
+// (about 8 us) behind the gather.  With a codec always (its tail kernel
+// needs the device copy); without one from kDeviceSlotBytes per batch on.
+constexpr uint64_t kDeviceSlotBytes = 1ull << 20;
+inline bool delivery_through_device(const tile_stream_configuration& cfg, const StreamPlan& P)
+{
+  return cfg.codec.id != CODEC_NONE ||
+         uint64_t(P.K) * P.total_chunks * P.chunk_bytes >= kDeviceSlotBytes;
+}
+
 // Pinned staging slots of a stream.
 constexpr uint64_t kStreamStageSlots = 4;
 

@@ -138,6 +138,7 @@ int Stream::init(const tile_stream_configuration* c, shard_sink* sk)
     CK(cudaEventCreateWithFlags(&ev_batch[i], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_codec_done[i], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&ev_agg_done[i], cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&ev_index_done[i], cudaEventDisableTiming));
     CK(cudaEventRecord(ev_agg_done[i], s_comp));
     CK(cudaEventRecord(ev_codec_done[i], s_enc[i]));
     CK(cudaMalloc(&d_epoch[i], round_up(P.epoch_bytes, 256) + 256));
@@ -419,6 +420,7 @@ void Stream::build_luts(int l,
 int Stream::setup_aggregate()
 {
   uint64_t max_positions = 0;
+  slots_on_device = delivery_through_device(cfg, P);
   for (int l = 0; l < P.nlod; ++l) {
     const LevelPlan& V = P.lv[l];
     const uint32_t slots = std::max<uint32_t>(V.batch_active, 1);
@@ -458,9 +460,7 @@ int Stream::setup_aggregate()
       CK(cudaMalloc(&D.d_offsets, (positions + 1) * 8));
       CK(cudaMalloc(&D.real_sizes, positions * 8 + 8));
       CK(cudaHostAlloc(&D.data, data, cudaHostAllocMapped));
-      // compressed batches are gathered in device memory and copied to the
-      // host by the copy engine (faster than SM stores over the link)
-      if (cfg.codec.id != CODEC_NONE)
+      if (slots_on_device)
         CK(cudaMalloc(&D.d_data, data));
     }
     // shard state (src/zarr/shard_delivery.c:10-34); the index lives on
@@ -545,6 +545,8 @@ void Stream::release()
       cudaEventDestroy(ev_codec_done[i]);
     if (ev_agg_done[i])
       cudaEventDestroy(ev_agg_done[i]);
+    if (ev_index_done[i])
+      cudaEventDestroy(ev_index_done[i]);
   }
   if (s_agg)
     cudaStreamDestroy(s_agg);
@@ -869,7 +871,6 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
     A.real_sizes = D.real_sizes;
     A.out = D.d_data ? D.d_data : D.data;
     D.positions = A.positions;
-    D.copied = 0;
     // the batch's runs of epochs per shard epoch, as delivery splits them
     // (src/zarr/shard_delivery.c:105-204)
     D.n_runs = 0;
@@ -908,6 +909,9 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
   if (timed_begin(sa, &metrics.aggregate, 0, 0))
     return 1;
   CK(launch_aggregate(ab, d_agg_scratch + si * agg_scratch_slot, sa));
+  if (timed_end(sa))
+    return 1;
+  CK(cudaEventRecord(ev_agg_done[si], sa)); // the compressed slots are free
   // the shard index entries of the batch and the index blobs (with their
   // crc32c) of every shard epoch it completes
   {
@@ -935,33 +939,26 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
     }
     CK(launch_index(ib, sa));
   }
-  // to the host: the expected bytes by the copy engine, the rest (if the
-  // batch is larger: the first batch, or a less compressible one) by a
-  // kernel that reads the total on the device -- no host wait either way
-  TailCopies tails{};
-  uint64_t tail_max = 0;
-  for (int k = 0; k < S.n_levels; ++k) {
-    DeliverySlot::Level& D = S.lv[S.level_of[k]];
-    if (!D.d_data)
-      continue;
-    D.copied = std::min(agg_estimate[S.level_of[k]], D.data_cap);
-    if (D.copied)
-      CK(cudaMemcpyAsync(D.data, D.d_data, D.copied, cudaMemcpyDeviceToHost, sa));
-    if (D.copied < D.data_cap) {
-      TailCopy& t = tails.lv[tails.n++];
-      t.dst = D.data;
-      t.src = D.d_data;
-      t.total = D.d_offsets + D.positions; // written by the aggregation
-      t.extra = cfg.shard_alignment;     // the zeroed slack after the batch
-      t.start = D.copied;
-      tail_max = std::max(tail_max, D.data_cap - D.copied);
+  cudaStream_t so = sa;
+  if (slots_on_device) {
+    // The copies run on the slot's encoder stream, beside the index kernel
+    // and the next batch's layout and gather (or, without a codec, its
+    // epochs): nothing else is queued there until the batch is delivered.
+    // A stream of a server keeps to its aggregation stream: many streams
+    // share the device's hardware queues, and one more of them in use was
+    // not faster there.
+    const bool apart = !engine;
+    if (apart) {
+      so = se;
+      CK(cudaEventRecord(ev_index_done[si], sa));
+      CK(cudaStreamWaitEvent(so, ev_agg_done[si], 0));
     }
+    if (copy_out(S, so))
+      return 1;
+    if (apart)
+      CK(cudaStreamWaitEvent(so, ev_index_done[si], 0));
   }
-  CK(launch_tail_copy(tails, tail_max, sa));
-  if (timed_end(sa))
-    return 1;
-  CK(cudaEventRecord(ev_agg_done[si], sa));
-  CK(cudaEventRecord(ev_batch[si], sa));
+  CK(cudaEventRecord(ev_batch[si], so));
   S.busy = 1;
   S.seq = ++batch_seq;
   S.epoch_done_ms.swap(pending_epoch_ms);
@@ -969,6 +966,47 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
   next_slot ^= 1;
   pool_claimed = false;
   return 0;
+}
+
+// A batch's shard-ordered bytes from the device copy of its delivery slot to
+// the host.  Without a codec the sizes are known (every chunk whole, a
+// shard group padded by less than the alignment): the copy engine moves all
+// of it.  With one, it moves the expected bytes, and a kernel that reads the
+// total on the device the rest (the first batch, or a less compressible
+// one) -- no host wait either way.
+int Stream::copy_out(DeliverySlot& S, cudaStream_t st)
+{
+  const uint64_t sa = cfg.shard_alignment;
+  TailCopies tails{};
+  uint64_t tail_max = 0, bytes = 0;
+  if (timed_begin(st, &metrics.d2h, 0, 0))
+    return 1;
+  for (int k = 0; k < S.n_levels; ++k) {
+    const int l = S.level_of[k];
+    const LevelPlan& V = P.lv[l];
+    DeliverySlot::Level& D = S.lv[l];
+    const bool known = cfg.codec.id == CODEC_NONE;
+    const uint64_t expect =
+      known ? uint64_t(S.active[l]) * V.layout.chunks_per_epoch * P.chunk_bytes +
+                (sa ? (V.covering / V.cps_inner + 1) * sa : 0)
+            : agg_estimate[l];
+    const uint64_t n = std::min(expect, D.data_cap);
+    if (n)
+      CK(cudaMemcpyAsync(D.data, D.d_data, n, cudaMemcpyDeviceToHost, st));
+    bytes += n;
+    if (!known && n < D.data_cap) {
+      TailCopy& t = tails.lv[tails.n++];
+      t.dst = D.data;
+      t.src = D.d_data;
+      t.total = D.d_offsets + D.positions; // written by the aggregation
+      t.extra = sa;                        // the zeroed slack after the batch
+      t.start = n;
+      tail_max = std::max(tail_max, D.data_cap - n);
+    }
+  }
+  CK(launch_tail_copy(tails, tail_max, st));
+  timers[timers_used - 1].in = timers[timers_used - 1].out = double(bytes);
+  return timed_end(st);
 }
 
 // Write one delivered batch to the shard sink

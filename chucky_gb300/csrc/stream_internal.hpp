@@ -36,10 +36,9 @@ struct DeliverySlot
     uint64_t* d_offsets = nullptr;  // [positions + 1]
     uint64_t* real_sizes = nullptr; // [positions], pre-padding
     uint8_t* data = nullptr;        // host (mapped) shard-ordered bytes
-    uint8_t* d_data = nullptr;      // device copy (compressed codecs)
+    uint8_t* d_data = nullptr;      // device copy (see slots_on_device)
     uint64_t positions_cap = 0, data_cap = 0;
     uint64_t positions = 0;         // of the batch in the slot
-    uint64_t copied = 0;            // bytes already copied to the host
     // shard index: the batch's runs of active epochs (host-written, read
     // by the index kernel) and the final index blobs of the shard epochs
     // the batch completes (written by the index kernel)
@@ -101,11 +100,11 @@ struct Stream
   uint8_t* d_pool = nullptr;
   uint64_t pool_half_bytes = 0; // 0: one pool (no codec)
   bool pool_claimed = false;    // the filling half waited for its last encode
-  cudaStream_t s_enc[2] = {}; // encoders, one stream per delivery slot
+  cudaStream_t s_enc[2] = {}; // encoders and copies out, one per delivery slot
   cudaEvent_t ev_pool_ready = nullptr;
   uint8_t* d_comp[2] = {}; // compressed slots, one per delivery slot
-  cudaStream_t s_agg = nullptr; // aggregation (host-link bound) stream
-  cudaEvent_t ev_codec_done[2] = {}, ev_agg_done[2] = {};
+  cudaStream_t s_agg = nullptr; // aggregation (a server's: and copies out)
+  cudaEvent_t ev_codec_done[2] = {}, ev_agg_done[2] = {}, ev_index_done[2] = {};
   uint64_t* d_sizes[2] = {}; // compressed sizes, one per delivery slot
   uint64_t comp_stride = 0;
   void* codec_state[2] = {}; // encoder scratch, one per delivery slot
@@ -164,6 +163,7 @@ struct Stream
   uint64_t agg_prev_total[LOD_MAX_LEVELS] = {}; // the batch before the last
   uint64_t agg_scratch_slot = 0; // entries per delivery slot
   DeliverySlot slot[2];
+  bool slots_on_device = false; // batches are gathered on the device first
   cudaEvent_t ev_batch[2] = {};
   int next_slot = 0;
   uint64_t batch_seq = 0;
@@ -219,6 +219,7 @@ struct Stream
   int run_epoch(uint64_t present);
   int kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks);
   int batch_boundary();
+  int copy_out(DeliverySlot& S, cudaStream_t st);
   int deliver(int si);
   int drain_all();
   int deliver_ready(); // deliver the batches the GPU has finished, in order
