@@ -4,15 +4,38 @@
 // LZ4_decompress_safe and the known chunk size (src/cpu/compress.c:85,
 // tests/test_compress_cpu.c:75-190); this is the same contract on the GPU.
 //
-// A warp per block.  Every lane parses the same token stream (the byte
-// loads broadcast within the warp), so the parse state needs no shuffles;
-// literals are copied with the lanes side by side, and a match of offset d
-// writes out[op + j] = out[op - d + j mod d] for j in [0, length), which
-// reads only bytes already final before op, so any offset, overlapping
-// ones included, is one pass.  Every read is checked against the block's
-// size and every write against the chunk size; a malformed block sets its
-// status and stops, nothing is read or written out of bounds.
+// A CTA per block, a tile of the block at a time.  The format is a chain of
+// tokens, each known only once the one before it is, and every match reads
+// bytes that earlier sequences wrote; decoded token by token a warp spends
+// about 500 cycles of memory latency on each.  Here both chains are
+// followed by all threads at once, in shared memory:
+//   parse  : for every byte of a window of the compressed block, where the
+//            next token would start if a token started there; exits of
+//            32-byte pieces by doubling within a warp (shuffles), of
+//            512-byte pieces by hops over those, so that the true chain
+//            crosses the window in one hop per warp; the tokens on it are
+//            then listed in order;
+//   place  : prefix sums of the sequences' lengths give each its place in
+//            an output tile;
+//   resolve: every output byte starts as a literal's value, a byte of the
+//            output before the tile, or a reference to a byte of the tile;
+//            references are followed by doubling (a byte takes its
+//            source's value or its source's reference), so a chain of d
+//            matches takes log2(d) rounds; a match that overlaps itself
+//            refers to its first period, one step deep;
+//   store  : the tile leaves with aligned 16-byte stores.
+// A sequence that does not fit a tile or whose length bytes run on (long
+// literal runs, long matches) is copied by the whole CTA.
+//
+// Bound by latency and the instructions of the parse (about 10 us for a
+// 16 KiB tile), not by memory.
+//
+// Every read is checked against the block's size and every write against
+// the chunk size.  A block the fast path cannot finish is decoded once more
+// by one warp, sequence by sequence, which sets its status; nothing is read
+// or written out of bounds.
 #include "chucky_gb300.h"
+#include "copy.cuh"
 #include "kernels_codec.hpp"
 #include "launch.cuh"
 
@@ -21,8 +44,6 @@
 namespace chucky {
 
 namespace {
-
-constexpr int kDecodeWarps = 4;
 
 enum : uint32_t
 {
@@ -33,23 +54,16 @@ enum : uint32_t
   kDecodeShort = 4,     // the block ends before the chunk is complete
 };
 
-__global__ void __launch_bounds__(32 * kDecodeWarps)
-lz4_decode_k(const uint8_t* in,
-             const uint64_t* in_off,
-             const uint64_t* in_size,
-             uint64_t n_chunks,
-             uint8_t* out,
-             uint64_t out_stride,
-             uint64_t chunk_bytes,
-             uint32_t* status)
+// One block by one warp.  Every lane parses the same tokens (the byte loads
+// broadcast within the warp); literals are copied side by side, and a match
+// of offset d writes out[op + j] = out[op - d + j mod d] for j in
+// [0, length), which reads only bytes already final before op.
+__device__ uint32_t lz4_decode_serial(const uint8_t* src,
+                                      uint64_t n,
+                                      uint8_t* dst,
+                                      uint64_t chunk_bytes,
+                                      int lane)
 {
-  const int lane = threadIdx.x & 31;
-  const uint64_t c = uint64_t(blockIdx.x) * kDecodeWarps + (threadIdx.x >> 5);
-  if (c >= n_chunks)
-    return; // the whole warp
-  const uint8_t* src = in + in_off[c];
-  const uint64_t n = in_size[c];
-  uint8_t* dst = out + c * out_stride;
   uint64_t ip = 0, op = 0;
   uint32_t st = kDecodeOk;
   while (true) {
@@ -124,9 +138,535 @@ lz4_decode_k(const uint8_t* in,
   }
   if (st == kDecodeOk && op != chunk_bytes)
     st = kDecodeShort;
-  if (lane == 0)
-    status[c] = st;
+  return st;
 }
+
+// ---- the tiled decoder -------------------------------------------------------
+
+constexpr uint32_t kPer = 16;       // window positions / tile bytes per thread
+constexpr uint32_t kWarpSpan = 512; // window positions per warp
+static_assert(kWarpSpan == 32 * kPer, "a warp's threads share its span");
+// length bytes of one field followed inside a window (each adds 255)
+constexpr uint32_t kMaxExt = 32;
+// where the chain goes from a position: the next token's position, or
+constexpr uint32_t kStop = 0x8000;  // | position: that token is not complete here
+constexpr uint32_t kEnd = 0xFFFE;   // the block's last sequence
+
+// One sequence of a tile.
+struct LzTok
+{
+  uint16_t out;  // place of its first byte in the tile
+  uint16_t src;  // window position of its literals
+  uint16_t lit;  // literals
+  uint16_t off;  // match offset (0: none, the last sequence)
+};
+
+template<int NT>
+struct LzShared
+{
+  static constexpr uint32_t kWindow = NT * kPer;
+  static constexpr uint32_t kTile = NT * kPer;
+  static constexpr uint32_t kWarps = NT / 32;
+  alignas(16) uint8_t win[kWindow + 16]; // compressed bytes (16-byte phase kept)
+  union
+  {
+    struct
+    {
+      uint16_t next[kWindow]; // chain step of every position
+      uint16_t exit[kWindow]; // where it leaves the position's 32-byte piece
+    } p;
+    struct
+    {
+      alignas(16) uint16_t ref[kTile + 16]; // value | 0x8000, or a tile index
+      LzTok tok[kWindow / 3 + 2];           // (a sequence takes >= 3 bytes)
+    } t;
+  };
+  uint32_t mask[NT / 2];      // tokens among 32 window positions each
+  uint16_t mask_at[NT / 2];   // tokens before them
+  uint32_t start[NT / 2 + 1]; // sequences starting among 32 tile bytes each
+  uint16_t start_at[NT / 2 + 1];
+  uint16_t exit2[kWarps][32]; // where a span's first 32 positions leave it
+  uint16_t entry[kWarps];     // the chain's first position in each span
+  uint32_t warp_sum[kWarps];
+  uint32_t chain_end;         // where the chain left the window (as `next`)
+  uint32_t cut, cut_pos, cut_out; // first sequence past the tile
+  uint32_t found;             // (long sequences) first byte that is not 255
+  uint32_t bad;
+};
+
+// Exclusive prefix sum over the CTA (one value per thread); `total` for all.
+template<int NT>
+__device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t* warp_sum, uint32_t& total)
+{
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o)
+      x += y;
+  }
+  __syncthreads(); // the sums' last readers
+  if (lane == 31)
+    warp_sum[warp] = x;
+  __syncthreads();
+  uint32_t t = lane < NT / 32 ? warp_sum[lane] : 0;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+    if (lane >= o)
+      t += y;
+  }
+  total = __shfl_sync(0xffffffffu, t, 31);
+  const uint32_t before = __shfl_sync(0xffffffffu, t, warp ? warp - 1 : 0);
+  return (warp ? before : 0) + x - v;
+}
+
+// The sequence at window position p: its literals and match, and the chain
+// step (the return value).
+__device__ __forceinline__ uint32_t lz4_step(const uint8_t* b,
+                                             uint32_t p,
+                                             uint32_t wlen,
+                                             bool at_end,
+                                             uint32_t& src,
+                                             uint32_t& lit,
+                                             uint32_t& ml,
+                                             uint32_t& off)
+{
+  const uint32_t t = b[p];
+  uint32_t q = p + 1;
+  lit = t >> 4;
+  if (lit == 15) {
+    for (uint32_t c = 0;; ++c) {
+      if (q >= wlen || c == kMaxExt)
+        return kStop | p;
+      const uint32_t x = b[q++];
+      lit += x;
+      if (x != 255)
+        break;
+    }
+  }
+  src = q;
+  q += lit;
+  off = 0;
+  ml = 0;
+  if (at_end && q == wlen)
+    return kEnd;
+  if (q + 2 > wlen)
+    return kStop | p;
+  off = uint32_t(b[q]) | uint32_t(b[q + 1]) << 8;
+  q += 2;
+  ml = (t & 15) + 4;
+  if (ml == 19) {
+    for (uint32_t c = 0;; ++c) {
+      if (q >= wlen || c == kMaxExt)
+        return kStop | p;
+      const uint32_t x = b[q++];
+      ml += x;
+      if (x != 255)
+        break;
+    }
+  }
+  return q;
+}
+
+// copy_bytes for a source with nothing readable past its end
+__device__ __forceinline__ void copy_exact(uint8_t* dst,
+                                           const uint8_t* src,
+                                           uint64_t n,
+                                           unsigned lane,
+                                           unsigned lanes)
+{
+  const uint64_t body = n > 64 ? n - 32 : 0; // (copy_bytes reads < 24 bytes on)
+  if (body)
+    copy_bytes(dst, src, body, lane, lanes);
+  for (uint64_t j = body + lane; j < n; j += lanes)
+    dst[j] = src[j];
+}
+
+// The length bytes at ip of a field that is already at its nibble's limit,
+// by the whole CTA; false when the block ends inside them.
+template<int NT>
+__device__ bool lz4_long_length(LzShared<NT>& S,
+                                const uint8_t* src,
+                                uint64_t n,
+                                uint64_t& ip,
+                                uint64_t& len)
+{
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0)
+      S.found = NT;
+    __syncthreads();
+    const uint64_t at = ip + threadIdx.x;
+    if (at >= n || src[at] != 255)
+      atomicMin(&S.found, threadIdx.x);
+    __syncthreads();
+    const uint32_t f = S.found;
+    len += uint64_t(f) * 255;
+    ip += f;
+    if (f < uint32_t(NT))
+      break;
+  }
+  if (ip >= n)
+    return false;
+  len += src[ip++];
+  return true;
+}
+
+// One sequence of any length at ip, by the whole CTA; false: malformed.
+template<int NT>
+__device__ bool lz4_long_sequence(LzShared<NT>& S,
+                                  const uint8_t* src,
+                                  uint64_t n,
+                                  uint8_t* dst,
+                                  uint64_t chunk_bytes,
+                                  uint64_t& ip,
+                                  uint64_t& op,
+                                  bool& last)
+{
+  const unsigned tid = threadIdx.x;
+  if (ip >= n)
+    return false;
+  const uint32_t token = src[ip++];
+  uint64_t lit = token >> 4;
+  if (lit == 15 && !lz4_long_length(S, src, n, ip, lit))
+    return false;
+  if (lit > n - ip || lit > chunk_bytes - op)
+    return false;
+  copy_exact(dst + op, src + ip, lit, tid, NT);
+  ip += lit;
+  op += lit;
+  last = ip == n;
+  if (last)
+    return true;
+  if (n - ip < 2)
+    return false;
+  const uint64_t off = uint64_t(src[ip]) | uint64_t(src[ip + 1]) << 8;
+  ip += 2;
+  uint64_t ml = (token & 15) + 4;
+  if (ml == 19 && !lz4_long_length(S, src, n, ip, ml))
+    return false;
+  if (off == 0 || off > op || ml > chunk_bytes - op)
+    return false;
+  __syncthreads(); // the literals
+  // the first 64 periods' bytes one by one, then copies of doubling length
+  // from the bytes already written (a multiple of the offset behind them)
+  uint64_t done = off * 64 < ml ? off * 64 : ml;
+  for (uint64_t j = tid; j < done; j += NT)
+    dst[op + j] = dst[op - off + (j < off ? j : uint32_t(j) % uint32_t(off))];
+  while (done < ml) {
+    __syncthreads();
+    const uint64_t k = done < ml - done ? done : ml - done;
+    copy_exact(dst + op + done, dst + op, k, tid, NT);
+    done += k;
+  }
+  op += ml;
+  __syncthreads();
+  return true;
+}
+
+// `n` bytes of a block at src by all NT threads; false when it is malformed.
+template<int NT>
+__device__ bool lz4_decode_tiles(LzShared<NT>& S,
+                                 const uint8_t* src,
+                                 const uint64_t n,
+                                 uint8_t* dst,
+                                 const uint64_t chunk_bytes)
+{
+  using Sh = LzShared<NT>;
+  constexpr unsigned kAll = 0xffffffffu;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  uint64_t ip = 0, op = 0;
+  uint32_t want = Sh::kWindow; // window bytes worth parsing
+  for (;;) {
+    if (ip >= n)
+      return false;
+    const uint32_t wlen = uint32_t(n - ip < want ? n - ip : want);
+    const bool at_end = ip + wlen == n;
+    // ---- the window, in the 16-byte phase of the block
+    const uint32_t sh = uint32_t(reinterpret_cast<uintptr_t>(src + ip) & 15);
+    const uint8_t* b = S.win + sh;
+    for (uint32_t v = tid; v * 16 < sh + wlen; v += NT) {
+      const uint32_t lo = v * 16, hi = lo + 16;
+      const uint8_t* g = src + ip + lo - sh; // (formed for the inner vectors)
+      if (lo >= sh && hi <= sh + wlen) {
+        *reinterpret_cast<uint4*>(S.win + lo) = *reinterpret_cast<const uint4*>(g);
+      } else {
+        for (uint32_t k = lo < sh ? sh : lo; k < hi && k < sh + wlen; ++k)
+          S.win[k] = src[ip + k - sh];
+      }
+    }
+    for (uint32_t i = tid; i < NT / 2 + 1; i += NT)
+      S.start[i] = 0;
+    if (tid == 0) {
+      S.cut = ~0u;
+      S.bad = 0;
+    }
+    __syncthreads();
+    // ---- chain steps and the exits of 32-byte pieces
+    const uint32_t w0 = warp * kWarpSpan;
+    if (w0 < wlen) {
+#pragma unroll 4
+      for (uint32_t i = 0; i < kPer; ++i) {
+        const uint32_t base = w0 + 32 * i, p = base + lane;
+        uint32_t a, l, m, o;
+        uint32_t j = p < wlen ? lz4_step(b, p, wlen, at_end, a, l, m, o) : (kStop | p);
+        S.p.next[p] = uint16_t(j);
+        // a piece holds at most 11 tokens: four doublings
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t r = __shfl_sync(kAll, j, int((j - base) & 31));
+          if (j - base < 32)
+            j = r;
+        }
+        S.p.exit[p] = uint16_t(j);
+      }
+      __syncwarp();
+      uint32_t e = w0 + lane;
+      do // (leaves the first piece, then hops over the others)
+        e = S.p.exit[e];
+      while (e < w0 + kWarpSpan && e < wlen);
+      S.exit2[warp][lane] = uint16_t(e);
+    }
+    __syncthreads();
+    // ---- the chain through the spans
+    if (tid == 0) {
+      uint32_t e = 0;
+      for (uint32_t w = 0; w < Sh::kWarps; ++w) {
+        const uint32_t hi = (w + 1) * kWarpSpan;
+        const bool in = e < hi && e < wlen;
+        S.entry[w] = uint16_t(in ? e : 0xFFFFu);
+        if (in) {
+          const uint32_t r = e - w * kWarpSpan;
+          if (r < 32)
+            e = S.exit2[w][r];
+          else
+            while (e < hi && e < wlen)
+              e = S.p.exit[e];
+        }
+      }
+      S.chain_end = e;
+    }
+    __syncthreads();
+    // ---- the tokens: each span's chain over its pieces, then each piece's
+    uint32_t mine = 0xFFFFu;
+    {
+      uint32_t e = S.entry[warp];
+      while (e < w0 + kWarpSpan && e < wlen) {
+        if (lane == ((e - w0) >> 5))
+          mine = e;
+        e = S.p.exit[e];
+      }
+    }
+    if (lane < kPer) {
+      uint32_t m = 0;
+      const uint32_t hi = w0 + 32 * (lane + 1);
+      for (uint32_t p = mine; p < hi && p < wlen;) {
+        const uint32_t x = S.p.next[p];
+        if (x >= kStop && x != kEnd)
+          break;
+        m |= 1u << (p & 31);
+        p = x;
+      }
+      S.mask[warp * kPer + lane] = m;
+    }
+    __syncthreads();
+    uint32_t ntok;
+    {
+      // two threads per piece: 16 positions each
+      const uint32_t half = (S.mask[tid >> 1] >> (16 * (tid & 1))) & 0xFFFFu;
+      const uint32_t at = cta_scan<NT>(__popc(half), S.warp_sum, ntok);
+      // parse them once more, now that they are tokens (the chain arrays'
+      // room is reused: everybody is past them)
+      uint32_t sum = 0, k = at, bits = half;
+      while (bits) {
+        const uint32_t p = (tid >> 1) * 32 + 16 * (tid & 1) + uint32_t(__ffs(int(bits)) - 1);
+        bits &= bits - 1;
+        uint32_t a = 0, l = 0, m = 0, o = 0;
+        const uint32_t x = lz4_step(b, p, wlen, at_end, a, l, m, o);
+        if (o == 0 && x != kEnd)
+          S.bad = 1; // (an offset of 0)
+        S.t.tok[k++] = LzTok{ uint16_t(l + m), uint16_t(a), uint16_t(l), uint16_t(o) };
+        sum += l + m;
+      }
+      uint32_t total;
+      uint32_t out = cta_scan<NT>(sum, S.warp_sum, total);
+      const uint32_t shd = uint32_t(reinterpret_cast<uintptr_t>(dst + op) & 15);
+      bits = half;
+      for (k = at; bits; ++k, bits &= bits - 1) {
+        const LzTok t = S.t.tok[k];
+        const uint32_t len = t.out;
+        if (out <= Sh::kTile && out + len > Sh::kTile) { // the first past the tile
+          S.cut = k;
+          S.cut_pos = (tid >> 1) * 32 + 16 * (tid & 1) + uint32_t(__ffs(int(bits)) - 1);
+          S.cut_out = out;
+        }
+        if (out + len <= Sh::kTile) {
+          S.t.tok[k].out = uint16_t(out);
+          if (t.off > op + out + t.lit)
+            S.bad = 1;
+          if (len)
+            atomicOr(&S.start[(out + shd) >> 5], 1u << ((out + shd) & 31));
+        }
+        out += len;
+      }
+      __syncthreads();
+      const bool cut = S.cut != ~0u;
+      const uint32_t chain_end = S.chain_end;
+      if (S.bad)
+        return false;
+      const uint32_t nout = cut ? S.cut_out : total;
+      const uint32_t used =
+        cut ? S.cut_pos
+            : (chain_end == kEnd ? wlen : (chain_end >= kStop ? chain_end - kStop : chain_end));
+      if (nout > chunk_bytes - op)
+        return false;
+      if (used == 0) { // a sequence that fits neither window nor tile
+        bool last = false;
+        if (!lz4_long_sequence(S, src, n, dst, chunk_bytes, ip, op, last))
+          return false;
+        if (last)
+          return op == chunk_bytes;
+        want = Sh::kWindow;
+        continue;
+      }
+      // ---- sequences before each 32 bytes of the tile
+      uint32_t dummy;
+      const uint32_t c = tid < NT / 2 ? uint32_t(__popc(S.start[tid])) : 0;
+      const uint32_t before = cta_scan<NT>(c, S.warp_sum, dummy);
+      if (tid < NT / 2)
+        S.start_at[tid] = uint16_t(before);
+      if (tid == NT / 2) // (the tile's phase makes it spill by < 16 bytes)
+        S.start_at[NT / 2] = uint16_t(before);
+      __syncthreads();
+      // ---- every byte's value or source.  (Zero-length last sequences have
+      // no start bit: they follow all others, so indices are unaffected.)
+      const uint32_t lim = shd + nout;
+      const uint8_t* done = dst + op;
+      uint32_t open = 0; // this thread's unresolved bytes
+#pragma unroll 4
+      for (uint32_t i = 0; i <= kPer; ++i) {
+        const uint32_t j = i * NT + tid;
+        if (j < shd || j >= lim)
+          continue;
+        const uint32_t w = j >> 5;
+        const uint32_t k =
+          S.start_at[w] + uint32_t(__popc(S.start[w] & (0xFFFFFFFFu >> (31 - (j & 31))))) - 1;
+        const LzTok t = S.t.tok[k];
+        const uint32_t r = j - shd - t.out;
+        uint32_t v;
+        if (r < t.lit) {
+          v = 0x8000u | b[t.src + r];
+        } else {
+          uint32_t m = r - t.lit;
+          if (m >= t.off)
+            m %= t.off;
+          const int32_t s = int32_t(uint32_t(t.out) + t.lit + m) - int32_t(t.off);
+          if (s < 0) {
+            v = 0x8000u | done[s];
+          } else {
+            v = uint32_t(s) + shd;
+            open |= 1u << i;
+          }
+        }
+        S.t.ref[j] = uint16_t(v);
+      }
+      // ---- follow the references
+      while (__syncthreads_or(open != 0)) {
+        for (uint32_t m = open; m; m &= m - 1) {
+          const uint32_t i = uint32_t(__ffs(int(m)) - 1), j = i * NT + tid;
+          const uint16_t v = S.t.ref[S.t.ref[j]];
+          S.t.ref[j] = v;
+          if (v & 0x8000u)
+            open &= ~(1u << i);
+        }
+      }
+      // ---- store
+      uint8_t* const o16 = dst + op - shd;
+      for (uint32_t v = tid; v * 16 < lim; v += NT) {
+        const uint32_t lo = v * 16;
+        if (lo >= shd && lo + 16 <= lim) {
+          const uint4 x = reinterpret_cast<const uint4*>(S.t.ref)[2 * v];
+          const uint4 y = reinterpret_cast<const uint4*>(S.t.ref)[2 * v + 1];
+          auto two = [](uint32_t a, uint32_t c2) { // four values of 16 bits -> 4 bytes
+            return (a & 0xFFu) | ((a >> 8) & 0xFF00u) | ((c2 & 0xFFu) << 16) |
+                   ((c2 & 0xFF0000u) << 8);
+          };
+          *reinterpret_cast<uint4*>(o16 + lo) =
+            make_uint4(two(x.x, x.y), two(x.z, x.w), two(y.x, y.y), two(y.z, y.w));
+        } else {
+          for (uint32_t k = lo < shd ? shd : lo; k < lo + 16 && k < lim; ++k)
+            dst[op + k - shd] = uint8_t(S.t.ref[k]);
+        }
+      }
+      ip += used;
+      op += nout;
+      if (!cut && chain_end == kEnd)
+        return op == chunk_bytes;
+      // a well compressed block fills the tile from part of the window:
+      // parse about as much next time
+      const uint32_t next = cut ? used + used / 4 + kWarpSpan : 2 * wlen;
+      want = next < Sh::kWindow ? next : Sh::kWindow;
+    }
+    __syncthreads(); // the tile is final and the shared arrays free
+  }
+}
+
+template<int NT>
+__global__ void __launch_bounds__(NT)
+lz4_decode_k(const uint8_t* in,
+             const uint64_t* in_off,
+             const uint64_t* in_size,
+             uint64_t n_chunks,
+             uint8_t* out,
+             uint64_t out_stride,
+             uint64_t chunk_bytes,
+             uint32_t* status)
+{
+  CHUCKY_DYN_SHARED(uint4, sm);
+  LzShared<NT>& S = *reinterpret_cast<LzShared<NT>*>(sm);
+  for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+    const uint8_t* src = in + in_off[c];
+    const uint64_t n = in_size[c];
+    uint8_t* dst = out + c * out_stride;
+    const bool ok = lz4_decode_tiles<NT>(S, src, n, dst, chunk_bytes);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      const uint32_t st =
+        ok ? uint32_t(kDecodeOk) : lz4_decode_serial(src, n, dst, chunk_bytes, int(threadIdx.x));
+      if (threadIdx.x == 0)
+        status[c] = st;
+    }
+    __syncthreads();
+  }
+}
+
+template<int NT>
+cudaError_t launch_lz4_decode_nt(const uint8_t* in,
+                                 const uint64_t* in_off,
+                                 const uint64_t* in_size,
+                                 uint64_t n_chunks,
+                                 uint8_t* out,
+                                 uint64_t out_stride,
+                                 uint64_t chunk_bytes,
+                                 uint32_t* status,
+                                 cudaStream_t st)
+{
+  constexpr size_t smem = sizeof(LzShared<NT>);
+  const cudaError_t e = cudaFuncSetAttribute(
+    lz4_decode_k<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (e != cudaSuccess)
+    return e;
+  const uint64_t grid = n_chunks < 0x7FFFFFFFull ? n_chunks : 0x7FFFFFFFull;
+  CHUCKY_LAUNCH(lz4_decode_k<NT>, unsigned(grid), NT, smem, st, in, in_off, in_size, n_chunks,
+                out, out_stride, chunk_bytes, status);
+  note_launches(1);
+  return cudaGetLastError();
+}
+
+// largest chunk of the 256-thread form
+constexpr uint64_t kSmallChunk = 16 << 10;
 
 } // namespace
 
@@ -140,11 +680,14 @@ cudaError_t launch_lz4_decode(const uint8_t* in,
                               uint32_t* status,
                               cudaStream_t st)
 {
-  const uint64_t grid = (n_chunks + kDecodeWarps - 1) / kDecodeWarps;
-  CHUCKY_LAUNCH(lz4_decode_k, unsigned(grid), 32 * kDecodeWarps, 0, st, in, in_off,
-                in_size, n_chunks, out, out_stride, chunk_bytes, status);
-  note_launches(1);
-  return cudaGetLastError();
+  // Chunks of up to 16 KiB: more CTAs of fewer threads, whose smaller tiles
+  // suit them; larger ones: as many threads per tile as a CTA holds, since a
+  // chunk's tiles follow one another.
+  return chunk_bytes <= kSmallChunk
+           ? launch_lz4_decode_nt<256>(in, in_off, in_size, n_chunks, out, out_stride,
+                                       chunk_bytes, status, st)
+           : launch_lz4_decode_nt<1024>(in, in_off, in_size, n_chunks, out, out_stride,
+                                        chunk_bytes, status, st);
 }
 
 } // namespace chucky

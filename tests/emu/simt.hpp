@@ -107,6 +107,18 @@ inline void __syncthreads()
 {
   simt::cta->all->arrive_and_wait();
 }
+inline int __syncthreads_or(int pred)
+{
+  static std::atomic<int> any{ 0 };
+  if (pred)
+    any = 1;
+  __syncthreads();
+  const int r = any;
+  __syncthreads();
+  any = 0;
+  __syncthreads();
+  return r;
+}
 inline void __syncwarp(unsigned = 0xffffffffu)
 {
   simt::warp_sync();
