@@ -13,7 +13,7 @@ void note_launches(unsigned n);
 // Streaming multiprocessors of the current device.
 int device_sm_count();
 
-// Raw LZ4 blocks back to chunk bytes (a warp per block, bounds-checked):
+// Raw LZ4 blocks back to chunk bytes (a CTA per block, bounds-checked):
 // block i is in_size[i] bytes at in + in_off[i] and decodes to chunk_bytes
 // bytes at out + i * out_stride; status[i] 0 when it did exactly that.
 cudaError_t launch_lz4_decode(const uint8_t* in,
@@ -34,7 +34,7 @@ struct ChunkRef
   uint64_t* size;    // compressed size (written)
 };
 
-// zstd frames back to chunk bytes (a CTA per frame, bounds-checked): frame
+// zstd frames back to chunk bytes (block-parallel, bounds-checked): frame
 // i is in_size[i] bytes at in + in_off[i] and decodes to chunk_bytes bytes
 // at out + i * out_stride; status[i] 0 when it did exactly that.
 cudaError_t launch_zstd_decode(const uint8_t* in,

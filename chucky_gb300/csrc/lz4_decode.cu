@@ -17,27 +17,24 @@
 //            then listed in order;
 //   place  : prefix sums of the sequences' lengths give each its place in
 //            an output tile;
-//   resolve: every output byte starts as a literal's value, a byte of the
-//            output before the tile, or a reference to a byte of the tile;
-//            references are followed by doubling (a byte takes its
-//            source's value or its source's reference), so a chain of d
-//            matches takes log2(d) rounds; a match that overlaps itself
-//            refers to its first period, one step deep;
-//   store  : the tile leaves with aligned 16-byte stores.
+//   execute: every byte of the tile finds its value by following references
+//            to earlier bytes (lz_tile.cuh).
 // A sequence that does not fit a tile or whose length bytes run on (long
 // literal runs, long matches) is copied by the whole CTA.
 //
-// Bound by latency and the instructions of the parse (about 10 us for a
-// 16 KiB tile), not by memory.
+// Bound by the integer instructions of the parse and of the tiles (about 20
+// us for a 16 KiB tile: 5 chain steps, 2 chain, 5 sequences, 8 tile), not by
+// memory: 64 sensor chunks of 1 MiB take 1.39 ms (a warp per block, sequence
+// by sequence: 62.3 ms), 1,024 of 16 KiB 0.15 ms.
 //
 // Every read is checked against the block's size and every write against
 // the chunk size.  A block the fast path cannot finish is decoded once more
 // by one warp, sequence by sequence, which sets its status; nothing is read
 // or written out of bounds.
 #include "chucky_gb300.h"
-#include "copy.cuh"
 #include "kernels_codec.hpp"
 #include "launch.cuh"
+#include "lz_tile.cuh"
 
 #include <cuda_runtime.h>
 
@@ -152,22 +149,20 @@ constexpr uint32_t kMaxExt = 32;
 constexpr uint32_t kStop = 0x8000;  // | position: that token is not complete here
 constexpr uint32_t kEnd = 0xFFFE;   // the block's last sequence
 
-// One sequence of a tile.
+// One sequence of a tile, as tile_run wants it.
 struct LzTok
 {
-  uint16_t out;  // place of its first byte in the tile
-  uint16_t src;  // window position of its literals
-  uint16_t lit;  // literals
-  uint16_t off;  // match offset (0: none, the last sequence)
+  uint16_t bound; // (its bytes, until its place is known)
+  uint16_t off;   // (0: none, the last sequence)
+  int32_t dlit;   // (literals << 16 | the window position of the first)
 };
 
 template<int NT>
 struct LzShared
 {
   static constexpr uint32_t kWindow = NT * kPer;
-  static constexpr uint32_t kTile = NT * kPer;
   static constexpr uint32_t kWarps = NT / 32;
-  alignas(16) uint8_t win[kWindow + 16]; // compressed bytes (16-byte phase kept)
+  alignas(16) uint8_t win[kWindow + 32]; // compressed bytes (16-byte phase kept)
   union
   {
     struct
@@ -177,14 +172,11 @@ struct LzShared
     } p;
     struct
     {
-      alignas(16) uint16_t ref[kTile + 16]; // value | 0x8000, or a tile index
-      LzTok tok[kWindow / 3 + 2];           // (a sequence takes >= 3 bytes)
+      LzTile<NT> tile;
+      LzTok tok[kWindow / 3 + 3]; // (a sequence takes >= 3 bytes)
     } t;
   };
   uint32_t mask[NT / 2];      // tokens among 32 window positions each
-  uint16_t mask_at[NT / 2];   // tokens before them
-  uint32_t start[NT / 2 + 1]; // sequences starting among 32 tile bytes each
-  uint16_t start_at[NT / 2 + 1];
   uint16_t exit2[kWarps][32]; // where a span's first 32 positions leave it
   uint16_t entry[kWarps];     // the chain's first position in each span
   uint32_t warp_sum[kWarps];
@@ -194,36 +186,10 @@ struct LzShared
   uint32_t bad;
 };
 
-// Exclusive prefix sum over the CTA (one value per thread); `total` for all.
-template<int NT>
-__device__ __forceinline__ uint32_t cta_scan(uint32_t v, uint32_t* warp_sum, uint32_t& total)
-{
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o)
-      x += y;
-  }
-  __syncthreads(); // the sums' last readers
-  if (lane == 31)
-    warp_sum[warp] = x;
-  __syncthreads();
-  uint32_t t = lane < NT / 32 ? warp_sum[lane] : 0;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-    if (lane >= o)
-      t += y;
-  }
-  total = __shfl_sync(0xffffffffu, t, 31);
-  const uint32_t before = __shfl_sync(0xffffffffu, t, warp ? warp - 1 : 0);
-  return (warp ? before : 0) + x - v;
-}
-
 // The sequence at window position p: its literals and match, and the chain
-// step (the return value).
+// step (the return value).  Straight-line for the common lengths: the first
+// length byte of either field is loaded whether it is needed or not (the
+// window is padded), only a second one takes a loop.
 __device__ __forceinline__ uint32_t lz4_step(const uint8_t* b,
                                              uint32_t p,
                                              uint32_t wlen,
@@ -233,55 +199,42 @@ __device__ __forceinline__ uint32_t lz4_step(const uint8_t* b,
                                              uint32_t& ml,
                                              uint32_t& off)
 {
-  const uint32_t t = b[p];
-  uint32_t q = p + 1;
+  const uint32_t t = b[p], x = b[p + 1];
   lit = t >> 4;
+  src = p + 1;
   if (lit == 15) {
-    for (uint32_t c = 0;; ++c) {
-      if (q >= wlen || c == kMaxExt)
-        return kStop | p;
-      const uint32_t x = b[q++];
-      lit += x;
-      if (x != 255)
-        break;
+    lit += x;
+    ++src;
+    if (x == 255) {
+      uint32_t y = 255;
+      for (uint32_t c = 1; y == 255; ++c) {
+        if (src >= wlen || c == kMaxExt)
+          return kStop | p;
+        y = b[src++];
+        lit += y;
+      }
     }
   }
-  src = q;
-  q += lit;
-  off = 0;
-  ml = 0;
-  if (at_end && q == wlen)
-    return kEnd;
-  if (q + 2 > wlen)
-    return kStop | p;
-  off = uint32_t(b[q]) | uint32_t(b[q + 1]) << 8;
-  q += 2;
+  const uint32_t e = src + lit; // past the literals
+  off = ml = 0;
+  if (e + 2 > wlen)
+    return at_end && e == wlen ? kEnd : (kStop | p);
+  off = uint32_t(b[e]) | uint32_t(b[e + 1]) << 8;
   ml = (t & 15) + 4;
+  uint32_t q = e + 2;
   if (ml == 19) {
-    for (uint32_t c = 0;; ++c) {
+    uint32_t y = b[q++];
+    ml += y;
+    for (uint32_t c = 1; y == 255; ++c) {
       if (q >= wlen || c == kMaxExt)
         return kStop | p;
-      const uint32_t x = b[q++];
-      ml += x;
-      if (x != 255)
-        break;
+      y = b[q++];
+      ml += y;
     }
+    if (q > wlen)
+      return kStop | p;
   }
   return q;
-}
-
-// copy_bytes for a source with nothing readable past its end
-__device__ __forceinline__ void copy_exact(uint8_t* dst,
-                                           const uint8_t* src,
-                                           uint64_t n,
-                                           unsigned lane,
-                                           unsigned lanes)
-{
-  const uint64_t body = n > 64 ? n - 32 : 0; // (copy_bytes reads < 24 bytes on)
-  if (body)
-    copy_bytes(dst, src, body, lane, lanes);
-  for (uint64_t j = body + lane; j < n; j += lanes)
-    dst[j] = src[j];
 }
 
 // The length bytes at ip of a field that is already at its nibble's limit,
@@ -350,17 +303,7 @@ __device__ bool lz4_long_sequence(LzShared<NT>& S,
   if (off == 0 || off > op || ml > chunk_bytes - op)
     return false;
   __syncthreads(); // the literals
-  // the first 64 periods' bytes one by one, then copies of doubling length
-  // from the bytes already written (a multiple of the offset behind them)
-  uint64_t done = off * 64 < ml ? off * 64 : ml;
-  for (uint64_t j = tid; j < done; j += NT)
-    dst[op + j] = dst[op - off + (j < off ? j : uint32_t(j) % uint32_t(off))];
-  while (done < ml) {
-    __syncthreads();
-    const uint64_t k = done < ml - done ? done : ml - done;
-    copy_exact(dst + op + done, dst + op, k, tid, NT);
-    done += k;
-  }
+  cta_match<NT>(dst + op, off, ml);
   op += ml;
   __syncthreads();
   return true;
@@ -397,8 +340,8 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
           S.win[k] = src[ip + k - sh];
       }
     }
-    for (uint32_t i = tid; i < NT / 2 + 1; i += NT)
-      S.start[i] = 0;
+    if (lane == 0)
+      S.entry[warp] = 0xFFFFu;
     if (tid == 0) {
       S.cut = ~0u;
       S.bad = 0;
@@ -433,19 +376,18 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
     // ---- the chain through the spans
     if (tid == 0) {
       uint32_t e = 0;
-      for (uint32_t w = 0; w < Sh::kWarps; ++w) {
-        const uint32_t hi = (w + 1) * kWarpSpan;
-        const bool in = e < hi && e < wlen;
-        S.entry[w] = uint16_t(in ? e : 0xFFFFu);
-        if (in) {
-          const uint32_t r = e - w * kWarpSpan;
-          if (r < 32)
-            e = S.exit2[w][r];
-          else
-            while (e < hi && e < wlen)
-              e = S.p.exit[e];
+      do {
+        const uint32_t w = e / kWarpSpan, r = e % kWarpSpan;
+        S.entry[w] = uint16_t(e);
+        if (r < 32) {
+          e = S.exit2[w][r];
+        } else {
+          const uint32_t hi = (w + 1) * kWarpSpan;
+          do
+            e = S.p.exit[e];
+          while (e < hi && e < wlen);
         }
-      }
+      } while (e < wlen);
       S.chain_end = e;
     }
     __syncthreads();
@@ -476,7 +418,7 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
     {
       // two threads per piece: 16 positions each
       const uint32_t half = (S.mask[tid >> 1] >> (16 * (tid & 1))) & 0xFFFFu;
-      const uint32_t at = cta_scan<NT>(__popc(half), S.warp_sum, ntok);
+      const uint32_t at = cta_scan<NT>(uint32_t(__popc(half)), S.warp_sum, ntok);
       // parse them once more, now that they are tokens (the chain arrays'
       // room is reused: everybody is past them)
       uint32_t sum = 0, k = at, bits = half;
@@ -487,27 +429,29 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
         const uint32_t x = lz4_step(b, p, wlen, at_end, a, l, m, o);
         if (o == 0 && x != kEnd)
           S.bad = 1; // (an offset of 0)
-        S.t.tok[k++] = LzTok{ uint16_t(l + m), uint16_t(a), uint16_t(l), uint16_t(o) };
+        S.t.tok[++k] = LzTok{ uint16_t(l + m), uint16_t(o), int32_t(l << 16 | a) };
         sum += l + m;
       }
+      tile_clear(S.t.tile);
       uint32_t total;
       uint32_t out = cta_scan<NT>(sum, S.warp_sum, total);
       const uint32_t shd = uint32_t(reinterpret_cast<uintptr_t>(dst + op) & 15);
       bits = half;
       for (k = at; bits; ++k, bits &= bits - 1) {
-        const LzTok t = S.t.tok[k];
-        const uint32_t len = t.out;
-        if (out <= Sh::kTile && out + len > Sh::kTile) { // the first past the tile
+        const LzTok t = S.t.tok[k + 1];
+        const uint32_t len = t.bound, l = uint32_t(t.dlit) >> 16, a = uint32_t(t.dlit) & 0xFFFFu;
+        if (out <= LzTile<NT>::kBytes && out + len > LzTile<NT>::kBytes) { // first past the tile
           S.cut = k;
           S.cut_pos = (tid >> 1) * 32 + 16 * (tid & 1) + uint32_t(__ffs(int(bits)) - 1);
           S.cut_out = out;
         }
-        if (out + len <= Sh::kTile) {
-          S.t.tok[k].out = uint16_t(out);
-          if (t.off > op + out + t.lit)
+        if (out + len <= LzTile<NT>::kBytes) {
+          S.t.tok[k + 1].bound = uint16_t(shd + out + l);
+          S.t.tok[k + 1].dlit = int32_t(a) - int32_t(shd + out);
+          if (t.off > op + out + l)
             S.bad = 1;
           if (len)
-            atomicOr(&S.start[(out + shd) >> 5], 1u << ((out + shd) & 31));
+            tile_mark(S.t.tile, shd, out);
         }
         out += len;
       }
@@ -531,75 +475,8 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
         want = Sh::kWindow;
         continue;
       }
-      // ---- sequences before each 32 bytes of the tile
-      uint32_t dummy;
-      const uint32_t c = tid < NT / 2 ? uint32_t(__popc(S.start[tid])) : 0;
-      const uint32_t before = cta_scan<NT>(c, S.warp_sum, dummy);
-      if (tid < NT / 2)
-        S.start_at[tid] = uint16_t(before);
-      if (tid == NT / 2) // (the tile's phase makes it spill by < 16 bytes)
-        S.start_at[NT / 2] = uint16_t(before);
-      __syncthreads();
-      // ---- every byte's value or source.  (Zero-length last sequences have
-      // no start bit: they follow all others, so indices are unaffected.)
-      const uint32_t lim = shd + nout;
-      const uint8_t* done = dst + op;
-      uint32_t open = 0; // this thread's unresolved bytes
-#pragma unroll 4
-      for (uint32_t i = 0; i <= kPer; ++i) {
-        const uint32_t j = i * NT + tid;
-        if (j < shd || j >= lim)
-          continue;
-        const uint32_t w = j >> 5;
-        const uint32_t k =
-          S.start_at[w] + uint32_t(__popc(S.start[w] & (0xFFFFFFFFu >> (31 - (j & 31))))) - 1;
-        const LzTok t = S.t.tok[k];
-        const uint32_t r = j - shd - t.out;
-        uint32_t v;
-        if (r < t.lit) {
-          v = 0x8000u | b[t.src + r];
-        } else {
-          uint32_t m = r - t.lit;
-          if (m >= t.off)
-            m %= t.off;
-          const int32_t s = int32_t(uint32_t(t.out) + t.lit + m) - int32_t(t.off);
-          if (s < 0) {
-            v = 0x8000u | done[s];
-          } else {
-            v = uint32_t(s) + shd;
-            open |= 1u << i;
-          }
-        }
-        S.t.ref[j] = uint16_t(v);
-      }
-      // ---- follow the references
-      while (__syncthreads_or(open != 0)) {
-        for (uint32_t m = open; m; m &= m - 1) {
-          const uint32_t i = uint32_t(__ffs(int(m)) - 1), j = i * NT + tid;
-          const uint16_t v = S.t.ref[S.t.ref[j]];
-          S.t.ref[j] = v;
-          if (v & 0x8000u)
-            open &= ~(1u << i);
-        }
-      }
-      // ---- store
-      uint8_t* const o16 = dst + op - shd;
-      for (uint32_t v = tid; v * 16 < lim; v += NT) {
-        const uint32_t lo = v * 16;
-        if (lo >= shd && lo + 16 <= lim) {
-          const uint4 x = reinterpret_cast<const uint4*>(S.t.ref)[2 * v];
-          const uint4 y = reinterpret_cast<const uint4*>(S.t.ref)[2 * v + 1];
-          auto two = [](uint32_t a, uint32_t c2) { // four values of 16 bits -> 4 bytes
-            return (a & 0xFFu) | ((a >> 8) & 0xFF00u) | ((c2 & 0xFFu) << 16) |
-                   ((c2 & 0xFF0000u) << 8);
-          };
-          *reinterpret_cast<uint4*>(o16 + lo) =
-            make_uint4(two(x.x, x.y), two(x.z, x.w), two(y.x, y.y), two(y.z, y.w));
-        } else {
-          for (uint32_t k = lo < shd ? shd : lo; k < lo + 16 && k < lim; ++k)
-            dst[op + k - shd] = uint8_t(S.t.ref[k]);
-        }
-      }
+      // (a last sequence of no bytes follows all marked ones)
+      tile_run<NT, 6>(S.t.tile, S.warp_sum, S.t.tok, b, dst + op, nout);
       ip += used;
       op += nout;
       if (!cut && chain_end == kEnd)
@@ -665,7 +542,7 @@ cudaError_t launch_lz4_decode_nt(const uint8_t* in,
   return cudaGetLastError();
 }
 
-// largest chunk of the 256-thread form
+// largest chunk of the small form
 constexpr uint64_t kSmallChunk = 16 << 10;
 
 } // namespace
@@ -684,9 +561,9 @@ cudaError_t launch_lz4_decode(const uint8_t* in,
   // suit them; larger ones: as many threads per tile as a CTA holds, since a
   // chunk's tiles follow one another.
   return chunk_bytes <= kSmallChunk
-           ? launch_lz4_decode_nt<256>(in, in_off, in_size, n_chunks, out, out_stride,
+           ? launch_lz4_decode_nt<CHUCKY_DECODE_THREADS>(in, in_off, in_size, n_chunks, out, out_stride,
                                        chunk_bytes, status, st)
-           : launch_lz4_decode_nt<1024>(in, in_off, in_size, n_chunks, out, out_stride,
+           : launch_lz4_decode_nt<CHUCKY_LZ4_THREADS>(in, in_off, in_size, n_chunks, out, out_stride,
                                         chunk_bytes, status, st);
 }
 

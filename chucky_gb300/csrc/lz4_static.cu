@@ -22,6 +22,7 @@
 // share the array and race.
 #include "kernels_codec.hpp"
 #include "plan.hpp"
+#include "scratch.hpp"
 
 #include <cuda_runtime.h>
 
@@ -35,12 +36,6 @@ constexpr int kMaxCachedContexts = 64;
 
 __device__ __align__(256) unsigned char g_lz4_scratch[kStaticScratchBytes];
 
-// cuCtxGetCurrent and cuCtxGetId, fetched through the runtime so that the
-// library does not link libcuda itself (CUresult is an int-sized enum,
-// CUcontext a pointer).
-using CtxGetCurrentFn = int (*)(void**);
-using CtxGetIdFn = int (*)(void*, unsigned long long*);
-
 struct CachedScratch
 {
   unsigned long long ctx_id;
@@ -48,41 +43,8 @@ struct CachedScratch
 };
 
 std::mutex g_setup_mutex;
-CtxGetCurrentFn g_ctx_get_current = nullptr;
-CtxGetIdFn g_ctx_get_id = nullptr;
-bool g_driver_looked_up = false;
 CachedScratch g_cache[kMaxCachedContexts];
 int g_cache_used = 0;
-
-void* driver_entry(const char* name)
-{
-  void* fn = nullptr;
-  cudaDriverEntryPointQueryResult q{};
-  if (cudaGetDriverEntryPointByVersion(name, &fn, 12000, cudaEnableDefault, &q) !=
-        cudaSuccess ||
-      q != cudaDriverEntryPointSuccess) {
-    cudaGetLastError(); // clear a failed lookup
-    return nullptr;
-  }
-  return fn;
-}
-
-// The ID of the calling thread's current context, or 0 when there is none
-// or the driver cannot tell (IDs start at 1).
-unsigned long long current_context_id()
-{
-  if (!g_driver_looked_up) {
-    g_driver_looked_up = true;
-    g_ctx_get_current = reinterpret_cast<CtxGetCurrentFn>(driver_entry("cuCtxGetCurrent"));
-    g_ctx_get_id = reinterpret_cast<CtxGetIdFn>(driver_entry("cuCtxGetId"));
-  }
-  void* ctx = nullptr;
-  unsigned long long id = 0;
-  if (!g_ctx_get_current || !g_ctx_get_id || g_ctx_get_current(&ctx) != 0 || !ctx ||
-      g_ctx_get_id(ctx, &id) != 0)
-    return 0;
-  return id;
-}
 
 void* scratch_for_current_context()
 {
@@ -90,7 +52,7 @@ void* scratch_for_current_context()
   if (cudaGetDevice(&dev) != cudaSuccess)
     return nullptr;
   std::lock_guard<std::mutex> lock(g_setup_mutex);
-  unsigned long long id = current_context_id();
+  unsigned long long id = chucky::current_context_id();
   for (int i = 0; id && i < g_cache_used; ++i)
     if (g_cache[i].ctx_id == id)
       return g_cache[i].ptr;
@@ -105,7 +67,7 @@ void* scratch_for_current_context()
     return nullptr;
   }
   if (!id)
-    id = current_context_id();
+    id = chucky::current_context_id();
   if (!id) {
     std::fprintf(stderr,
                  "chucky_gb300: static LZ4 scratch: the current CUDA context of "

@@ -20,6 +20,7 @@
 //   batch:  src/cpu/pipeline.c:113-190, src/gpu/flush.compress_agg.c:224-371
 //   shards: src/zarr/shard_delivery.c:10-204
 #include "plan.hpp"
+#include "scratch.hpp"
 #include "stream_internal.hpp"
 
 #include <algorithm>
@@ -1496,6 +1497,7 @@ tile_stream_gpu_destroy(tile_stream_gpu* s)
     return;
   s->impl.release();
   delete s;
+  chucky::scratch_trim();
 }
 
 extern "C" stream_metrics

@@ -10,15 +10,18 @@
 // frames one after another.  Frames with a dictionary are reported as
 // unsupported; a content checksum is skipped, not verified.
 //
-// One CTA per chunk, its first thread decoding (the format is sequential
-// within a block); the decoding tables live in shared memory.  Literals are
-// Huffman-decoded on demand while the sequences execute (stream by stream,
-// in order), so no literal buffer is needed.  Every read is checked against
-// the chunk's compressed size and every write against chunk_bytes; a
-// malformed frame sets its status and stops.
+// Two decoders.  Frames are decoded block-parallel (zstd_decode_blocks.cuh);
+// the sequential decoder below takes what that leaves -- malformed chunks,
+// several or skippable frames, dictionary frames -- and every chunk when
+// there is no scratch for the lists: a CTA per chunk, its first thread
+// decoding, the tables in shared memory, literals Huffman-decoded on demand
+// while the sequences execute.  Every read is checked against the chunk's
+// compressed size and every write against chunk_bytes; a malformed frame
+// sets its status and stops.
 #include "chucky_gb300.h"
 #include "kernels_codec.hpp"
 #include "launch.cuh"
+#include "scratch.hpp"
 #include "zstd_format.cuh"
 
 #include <cuda_runtime.h>
@@ -667,16 +670,28 @@ __device__ uint32_t decode_block(const uint8_t* p, uint64_t n, Frame& F, DecShar
   return L.finished() ? kZOk : kZCorrupt;
 }
 
+} // namespace
+
+} // namespace chucky
+
+#include "zstd_decode_blocks.cuh"
+
+namespace chucky {
+
+namespace {
+
+// `frames`: only the chunks flagged there (null: all).
 __global__ void __launch_bounds__(32) zstd_decode_k(const uint8_t* in,
                                                     const uint64_t* in_off,
                                                     const uint64_t* in_size,
                                                     uint8_t* out,
                                                     uint64_t out_stride,
                                                     uint64_t chunk_bytes,
-                                                    uint32_t* status)
+                                                    uint32_t* status,
+                                                    const ZFrame* frames)
 {
   __shared__ DecShared S;
-  if (threadIdx.x != 0)
+  if (threadIdx.x != 0 || (frames && !frames[blockIdx.x].slow))
     return;
   const uint64_t c = blockIdx.x;
   const uint8_t* p = in + in_off[c];
@@ -830,10 +845,45 @@ cudaError_t launch_zstd_decode(const uint8_t* in,
 {
   if (!n_chunks)
     return cudaSuccess;
-  note_launches(1);
-  CHUCKY_LAUNCH(zstd_decode_k, unsigned(n_chunks), 32, 0, st, in, in_off, in_size, out,
-                out_stride, chunk_bytes, status);
-  return cudaGetLastError();
+  // chunks per launch set: as many as the kept scratch has lists for
+  const uint64_t one = zd_bytes(1, chunk_bytes);
+  uint64_t wave = kZdScratch / one;
+  wave = wave < 1 ? 1 : wave > n_chunks ? n_chunks : wave;
+  uint8_t* const scratch =
+    chunk_bytes < (1ull << 32)
+      ? static_cast<uint8_t*>(scratch_acquire(zd_bytes(wave, chunk_bytes), st))
+      : nullptr;
+  cudaError_t e = cudaSuccess;
+  if (!scratch) {
+    note_launches(1);
+    CHUCKY_LAUNCH(zstd_decode_k, unsigned(n_chunks), 32, 0, st, in, in_off, in_size, out,
+                  out_stride, chunk_bytes, status, static_cast<const ZFrame*>(nullptr));
+    return cudaGetLastError();
+  }
+  for (uint64_t f = 0; f < n_chunks && e == cudaSuccess; f += wave) {
+    ZWave W{};
+    W.in = in;
+    W.in_off = in_off + f;
+    W.in_size = in_size + f;
+    W.out = out + f * out_stride;
+    W.out_stride = out_stride;
+    W.chunk_bytes = chunk_bytes;
+    W.status = status + f;
+    W.n = n_chunks - f < wave ? n_chunks - f : wave;
+    W.max_blk = zd_max_blk(chunk_bytes);
+    W.max_seq = zd_max_seq(chunk_bytes);
+    W.seqs = reinterpret_cast<uint64_t*>(scratch);
+    W.blocks = reinterpret_cast<ZBlk*>(W.seqs + wave * W.max_seq);
+    W.frames = reinterpret_cast<ZFrame*>(W.blocks + wave * W.max_blk);
+    if ((e = zd_launch(W, st)) != cudaSuccess)
+      break;
+    note_launches(1);
+    CHUCKY_LAUNCH(zstd_decode_k, unsigned(W.n), 32, 0, st, in, W.in_off, W.in_size, W.out,
+                  out_stride, chunk_bytes, W.status, static_cast<const ZFrame*>(W.frames));
+    e = cudaGetLastError();
+  }
+  scratch_release(scratch, st);
+  return e;
 }
 
 } // namespace chucky

@@ -186,9 +186,14 @@ extern "C"
    * table, bitstream or offset, 3 when it would write past chunk_bytes, 4
    * when it decodes to fewer bytes, 5 for a dictionary frame; a malformed
    * frame is never read or written out of bounds.  Runs asynchronously on
-   * `cuda_stream` (a cudaStream_t; NULL for the default stream); a CTA per
-   * chunk, no scratch.  Returns 0 when launched, 1 for invalid arguments, 3
-   * for a CUDA error. */
+   * `cuda_stream` (a cudaStream_t; NULL for the default stream).  The
+   * blocks of a chunk are decoded side by side with device scratch from a
+   * pool of the library's own (about twice the output, 256 MiB at most at a
+   * time; what the pool keeps is handed back when a stream is destroyed);
+   * where there is none to be had -- no memory left, the stream being
+   * captured -- each chunk is decoded sequentially by one thread, with the
+   * same result.  Returns 0 when launched, 1 for invalid arguments, 3 for a
+   * CUDA error. */
   int chucky_zstd_decode_chunks(const void* d_in,
                                 const uint64_t* d_in_offsets,
                                 const uint64_t* d_in_sizes,

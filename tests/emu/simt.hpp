@@ -186,6 +186,11 @@ inline unsigned __funnelshift_r(unsigned lo, unsigned hi, unsigned s)
   const uint64_t v = (uint64_t(hi) << 32) | lo;
   return unsigned(v >> (s & 31));
 }
+inline unsigned __funnelshift_l(unsigned lo, unsigned hi, unsigned s)
+{
+  const uint64_t v = (uint64_t(hi) << 32) | lo;
+  return unsigned((v << (s & 31)) >> 32);
+}
 inline uint64_t __umul64hi(uint64_t a, uint64_t b)
 {
   return uint64_t((unsigned __int128)a * b >> 64);
@@ -263,6 +268,25 @@ inline cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t = null
   std::memset(p, v, n);
   return cudaSuccess;
 }
+
+// decoders' CTAs of one or two warps: quicker here, and more tiles per chunk
+#define CHUCKY_DECODE_THREADS 64
+#define CHUCKY_LZ4_THREADS 64
+#define CHUCKY_ZSTD_EXEC_THREADS 64
+#define CHUCKY_DECODE_WARPS 1
+
+// device scratch of a call (scratch.hpp)
+#define CHUCKY_SCRATCH_EMULATED
+namespace chucky {
+inline void* scratch_acquire(size_t n, cudaStream_t)
+{
+  return std::malloc(n);
+}
+inline void scratch_release(void* p, cudaStream_t)
+{
+  std::free(p);
+}
+} // namespace chucky
 
 enum cudaFuncAttribute
 {
