@@ -59,13 +59,16 @@ constexpr uint32_t kLz4WideBack = 3;
 constexpr int kLz4WideLog = 15;
 __host__ __device__ inline bool lz4_wide(int level) { return level >= 2; }
 
-// One CTA per region, a warp per segment of it.
-__global__ void __launch_bounds__(32 * kSegsPerRegion)
+// One CTA per region, a warp per segment of it.  kWide: the levels with the
+// wide window (a kernel of their own: its registers would cost the other
+// levels a quarter of their warps).
+template<bool kWide>
+__global__ void __launch_bounds__(32 * kSegsPerRegion, kWide ? kWideCtas : 1)
 lz4_find_k(CodecBatch b,
            Seq* seqs,
            SegMeta* meta,
            uint32_t regions_per_chunk,
-           const uint16_t* wide_tables) // null: the region's own window only
+           const uint16_t* wide_tables)
 {
   __shared__ __align__(16) uint16_t tables[kSegsPerRegion][1 << kHashLog];
   CHUCKY_DYN_SHARED(uint32_t, words); // kRegionStageWords
@@ -92,13 +95,13 @@ lz4_find_k(CodecBatch b,
   Seq* out = seqs + seg * kMaxSeqPerSeg;
   // the wide window: the 3 regions before (LZ4 offsets reach 65535 back)
   const WideWindow W{ base,
-                      wide_tables ? wide_tables + chunk * regions_per_chunk *
-                                                    wide_entries(kLz4WideLog)
-                                  : nullptr,
+                      kWide ? wide_tables + chunk * regions_per_chunk *
+                                              wide_entries(kLz4WideLog)
+                            : nullptr,
                       uint32_t(r0 / kRegionBytes), kLz4WideBack, 65535u, kLz4WideLog };
-  const SegInfo info = lz77_parse_segment(
+  const SegInfo info = lz77_parse_segment<kWide>(
     words, r0, s0, s1, start_limit, match_end, tables[w], out,
-    b.min_match > 4 ? uint32_t(b.min_match) : 4u, wide_tables ? &W : nullptr,
+    b.min_match > 4 ? uint32_t(b.min_match) : 4u, W,
     b.strength > 0 ? b.strength : kSearchStrength);
   __syncwarp();
   // encoded size of everything but sequence 0's literal part
@@ -351,9 +354,14 @@ cudaError_t launch_lz4(CodecBatch b, void* scratch, cudaStream_t st)
       return e;
   }
   note_launches(3);
-  CHUCKY_LAUNCH(lz4_find_k, unsigned(b.n_chunks * rpc), 32 * kSegsPerRegion,
-                kRegionStageWords * sizeof(uint32_t), st, b, seqs, meta, rpc,
-                static_cast<const uint16_t*>(wide));
+  constexpr size_t smem = kRegionStageWords * sizeof(uint32_t);
+  const unsigned regions = unsigned(b.n_chunks * rpc);
+  if (wide)
+    CHUCKY_LAUNCH(lz4_find_k<true>, regions, 32 * kSegsPerRegion, smem, st, b, seqs, meta, rpc,
+                  static_cast<const uint16_t*>(wide));
+  else
+    CHUCKY_LAUNCH(lz4_find_k<false>, regions, 32 * kSegsPerRegion, smem, st, b, seqs, meta, rpc,
+                  static_cast<const uint16_t*>(nullptr));
   if ((e = cudaGetLastError()) != cudaSuccess)
     return e;
   CHUCKY_LAUNCH(lz4_plan_k, unsigned((b.n_chunks + kWarps - 1) / kWarps), 32 * kWarps, 0,

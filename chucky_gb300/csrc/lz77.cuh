@@ -91,6 +91,11 @@ struct SegInfo
 // (hash log per codec: 15 bits for LZ4, 14 for zstd; the zstd parse reaches
 // further back, so smaller tables keep more of them in L2)
 __host__ __device__ constexpr uint64_t wide_entries(int hlog) { return uint64_t(1) << hlog; }
+// CTAs per SM the wide-window parse is compiled for.  Its probes live on what
+// the staged regions leave of the L1: 16 sensor chunks (4 MiB) at LZ4 level 2
+// take 2.08 ms with 7 CTAs (60 KB of L1 left) and 3.3-3.6 ms with 8 or 9 (28
+// KB), 64 cube chunks at zstd level 3 1.79 ms with 7, 2.36 ms with 8.
+constexpr int kWideCtas = 7;
 // lanes whose local match is shorter than this probe the wide window
 constexpr uint32_t kWideProbeBelow = 16;
 
@@ -224,7 +229,8 @@ struct WideLane
   bool on;        // still searching
   uint32_t q, x;  // position (region-relative) and its 4 bytes
   uint32_t h, tag;
-  uint32_t cap, need;
+  uint32_t cap, need; // longest match allowed, shortest taken
+  uint32_t x2;        // the 4 bytes that end at `need`
 };
 
 __device__ __forceinline__ WideLane wide_lane(const WideWindow& W,
@@ -233,16 +239,18 @@ __device__ __forceinline__ WideLane wide_lane(const WideWindow& W,
                                               uint32_t x,
                                               uint32_t end,
                                               bool ok,
-                                              uint32_t len)
+                                              uint32_t len,
+                                              const uint32_t* words)
 {
   WideLane L;
-  L.on = probe;
   L.q = q;
   L.x = x;
   L.h = hash4w(x, W.hlog);
   L.tag = wide_tag(x, W.hlog);
   L.cap = probe ? min(kLaneExtend - 1, end - q) : 0;
   L.need = ok ? len + 1 : 4;
+  L.on = probe && L.need <= L.cap;
+  L.x2 = L.on ? word_at(words, q + L.need - 4) : 0;
   return L;
 }
 
@@ -254,6 +262,14 @@ __device__ __forceinline__ WideLane wide_lane(const WideWindow& W,
 // `words`).  The two searches are independent; their loads are issued side
 // by side.  Where probing has thinned out (`step` > 1: a literal run) only
 // the two nearest regions are probed.
+//
+// Bound by the latency of its random loads and by instructions (half of the
+// issue slots).  64 cube chunks (512 KiB) at zstd level 3 take 1.79 ms (1.88
+// with every equal candidate measured where it was found), 16 sensor chunks
+// (4 MiB) 3.82 (4.02) ms; at LZ4 level 2, 2.08 (3.55) ms, most of it by the
+// CTAs per SM.  Loading several regions' entries or candidates ahead (1.56
+// ms of find kernel against 1.29) and one 16-byte entry for all regions of a
+// hash (1.47) were slower: their registers cost more warps than the loads.
 __device__ __forceinline__ void wide_probe2(const WideWindow& W,
                                             const uint32_t* words,
                                             uint32_t r0,
@@ -269,43 +285,63 @@ __device__ __forceinline__ void wide_probe2(const WideWindow& W,
 {
   const uint64_t entries = wide_entries(W.hlog);
   const uint32_t nb = min(step > 1 ? min(W.back, 2u) : W.back, W.region);
-  for (uint32_t k = 0; k < nb && (A.on || B.on); ++k) {
-    const uint32_t rr = W.region - 1 - k;
-    const uint16_t* tb = W.tables + uint64_t(rr) * entries;
-    const uint16_t ta = A.on ? tb[A.h] : uint16_t(0xFFFF);
-    const uint16_t tbb = B.on ? tb[B.h] : uint16_t(0xFFFF);
-    const bool ga = ta != 0xFFFF && (uint32_t(ta) >> 14) == A.tag;
-    const bool gb = tbb != 0xFFFF && (uint32_t(tbb) >> 14) == B.tag;
-    const uint32_t cxa = rr * kRegionBytes + (ta & 0x3FFFu);
-    const uint32_t cxb = rr * kRegionBytes + (tbb & 0x3FFFu);
-    // the regions further back are further still
-    const bool fa = ga && r0 + A.q - cxa > W.max_dist;
-    const bool fb = gb && r0 + B.q - cxb > W.max_dist;
-    if (fa)
-      A.on = false;
-    if (fb)
-      B.on = false;
-    const bool va = ga && !fa, vb = gb && !fb;
-    const uint32_t xa = va ? load4(W.chunk, cxa) : ~A.x;
-    const uint32_t xb = vb ? load4(W.chunk, cxb) : ~B.x;
-    if (va && xa == A.x) {
+  // A sweep takes every lane to its next candidate whose first 4 bytes match
+  // and the 4 that end at the length it must have (up to 8 bytes that is all
+  // of them); the lanes then measure theirs together (measured as each was
+  // found, lanes that find theirs in different regions took turns).  A lane
+  // whose candidate is not longer goes on behind it.
+  uint32_t ka = 0, kb = 0; // regions done
+  while (A.on || B.on) {
+    uint32_t cxa = 0, cxb = 0;
+    bool fa = false, fb = false; // found
+    for (uint32_t k = 0; k < nb && ((A.on && !fa) || (B.on && !fb)); ++k) {
+      const uint32_t rr = W.region - 1 - k;
+      const uint16_t* tb = W.tables + uint64_t(rr) * entries;
+      const bool sa = A.on && !fa && k >= ka, sb = B.on && !fb && k >= kb;
+      const uint32_t ta = sa ? tb[A.h] : 0xFFFFu;
+      const uint32_t tbb = sb ? tb[B.h] : 0xFFFFu;
+      const bool ga = ta != 0xFFFF && (ta >> 14) == A.tag;
+      const bool gb = tbb != 0xFFFF && (tbb >> 14) == B.tag;
+      const uint32_t pa = rr * kRegionBytes + (ta & 0x3FFFu);
+      const uint32_t pb = rr * kRegionBytes + (tbb & 0x3FFFu);
+      // the regions further back are further still
+      const bool xa = ga && r0 + A.q - pa > W.max_dist;
+      const bool xb = gb && r0 + B.q - pb > W.max_dist;
+      A.on = A.on && !xa;
+      B.on = B.on && !xb;
+      const uint32_t va = ga && !xa ? load4(W.chunk, pa) : ~A.x;
+      const uint32_t vb = gb && !xb ? load4(W.chunk, pb) : ~B.x;
+      if (va == A.x && (A.need == 4 || load4(W.chunk, pa + A.need - 4) == A.x2)) {
+        fa = true;
+        cxa = pa;
+        ka = k + 1;
+      }
+      if (vb == B.x && (B.need == 4 || load4(W.chunk, pb + B.need - 4) == B.x2)) {
+        fb = true;
+        cxb = pb;
+        kb = k + 1;
+      }
+    }
+    if (fa) {
       const uint32_t m = wide_extend(W, words, A.q, cxa, A.cap);
       if (m >= A.need) {
         oka = true;
         la = m;
         ca = cxa - r0; // before the region: wraps, offsets stay q - cand
-        A.on = false;
+        fa = false;
       }
     }
-    if (vb && xb == B.x) {
+    A.on = A.on && fa;
+    if (fb) {
       const uint32_t m = wide_extend(W, words, B.q, cxb, B.cap);
       if (m >= B.need) {
         okb = true;
         lb = m;
         cb = cxb - r0;
-        B.on = false;
+        fb = false;
       }
     }
+    B.on = B.on && fb;
   }
 }
 
@@ -313,8 +349,9 @@ __device__ __forceinline__ void wide_probe2(const WideWindow& W,
 // r0 <= s0) on are staged in `words`.  Matches may start at positions in
 // [s0, start_limit), reach back to r0 and end at or before `match_end`.
 // `table` holds 1 << kHashLog u16 entries private to this warp (16-byte
-// aligned).
-__device__ inline SegInfo lz77_parse_segment(const uint32_t* words,
+// aligned).  kWide: matches in the wide window `wide` too.
+template<bool kWide>
+__device__ __forceinline__ SegInfo lz77_parse_segment(const uint32_t* words,
                                              uint32_t r0,
                                              uint32_t s0,
                                              uint32_t s1,
@@ -322,9 +359,9 @@ __device__ inline SegInfo lz77_parse_segment(const uint32_t* words,
                                              uint32_t match_end,
                                              uint16_t* table,
                                              Seq* out,
-                                             uint32_t min_match = 4,
-                                             const WideWindow* wide = nullptr,
-                                             int strength = kSearchStrength)
+                                             uint32_t min_match,
+                                             const WideWindow& wide,
+                                             int strength)
 {
   const int lane = threadIdx.x & 31;
   const uint8_t* bytes = reinterpret_cast<const uint8_t*>(words);
@@ -478,11 +515,11 @@ __device__ inline SegInfo lz77_parse_segment(const uint32_t* words,
     }
     uint32_t la = oka ? lane_match(words, bytes, qa, ca, end) : 0;
     uint32_t lb = okb ? lane_match(words, bytes, qb, cb, end) : 0;
-    if (wide) { // earlier regions, for lanes without a good local match
+    if constexpr (kWide) { // earlier regions, for lanes without a good local match
       const bool pa = va && la < kWideProbeBelow, pb = vb && lb < kWideProbeBelow;
       if (pa || pb)
-        wide_probe2(*wide, words, r0, step, wide_lane(*wide, pa, qa, xa, end, oka, la), oka,
-                    ca, la, wide_lane(*wide, pb, qb, xb, end, okb, lb), okb, cb, lb);
+        wide_probe2(wide, words, r0, step, wide_lane(wide, pa, qa, xa, end, oka, la, words),
+                    oka, ca, la, wide_lane(wide, pb, qb, xb, end, okb, lb, words), okb, cb, lb);
     }
     __syncwarp();
     if (va)

@@ -212,19 +212,21 @@ __host__ __device__ inline bool zstd_wide(int level) { return level >= 3; }
 constexpr uint32_t kSeqHistML = 36, kSeqHistOF = 36 + 53, kSeqHistBad = 36 + 53 + 32;
 constexpr uint32_t kSeqHistWords = 128;
 
-__global__ void __launch_bounds__(32 * kSegsPerRegion)
+// (kWide as in lz4_find_k.)
+template<bool kWide>
+__global__ void __launch_bounds__(32 * kSegsPerRegion, kWide ? kWideCtas : 1)
 zstd_find_k(CodecBatch b,
             Seq* seqs,
             ZSeg* meta,
             uint32_t* chunk_hist,
             uint8_t* litbuf,
             uint32_t regions_per_chunk,
-            const uint16_t* wide_tables, // null: the region's own window only
-            uint32_t* seq_hist)          // null: no sequence-code histograms
+            const uint16_t* wide_tables,
+            uint32_t* seq_hist) // sequence-code histograms (kWide)
 {
   __shared__ __align__(16) uint16_t tables[kSegsPerRegion][1 << kHashLog];
   __shared__ uint32_t seg_nseq[kSegsPerRegion], seg_trail[kSegsPerRegion];
-  __shared__ uint32_t shist[kSeqHistWords];
+  __shared__ uint32_t shist[kWide ? kSeqHistWords : 1];
   CHUCKY_DYN_SHARED(uint32_t, words); // kRegionStageWords
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t chunk = blockIdx.x / regions_per_chunk;
@@ -240,26 +242,25 @@ zstd_find_k(CodecBatch b,
   SegInfo info{ 0, 0 };
   if (has) {
     const WideWindow W{ base,
-                        wide_tables ? wide_tables + chunk * regions_per_chunk *
-                                                      wide_entries(kZstdWideLog)
-                                    : nullptr,
+                        kWide ? wide_tables + chunk * regions_per_chunk *
+                                                wide_entries(kZstdWideLog)
+                              : nullptr,
                         uint32_t(r0 / kRegionBytes), kZstdWideBack,
                         (kZstdWideBack + 1) * kRegionBytes, kZstdWideLog };
-    const uint32_t mm = wide_tables ? kMinMatchWide
-                                    : (b.min_match >= 4 ? uint32_t(b.min_match) : kMinMatch);
-    info = lz77_parse_segment(words, r0, s0, s1, s1, s1, tables[w], out, mm,
-                              wide_tables ? &W : nullptr,
-                              b.strength > 0 ? b.strength : kSearchStrength);
+    const uint32_t mm =
+      kWide ? kMinMatchWide : (b.min_match >= 4 ? uint32_t(b.min_match) : kMinMatch);
+    info = lz77_parse_segment<kWide>(words, r0, s0, s1, s1, s1, tables[w], out, mm, W,
+                                     b.strength > 0 ? b.strength : kSearchStrength);
   }
   if (lane == 0) {
     seg_nseq[w] = info.nseq;
     seg_trail[w] = info.trailing;
   }
-  if (seq_hist)
+  if constexpr (kWide)
     for (int i = threadIdx.x; i < int(kSeqHistWords); i += blockDim.x)
       shist[i] = 0;
   __syncthreads(); // the region is no longer needed as history
-  if (seq_hist && has) {
+  if (kWide && has) {
     // codes of the segment's sequences (as the block kernel forms them:
     // the first takes the literals carried from the block's earlier
     // segments since its last sequence), counted per CTA
@@ -377,7 +378,7 @@ zstd_find_k(CodecBatch b,
         atomicOr(ch + i, t);
     }
   }
-  if (seq_hist) // the CTA's code counts, added to its chunk's
+  if constexpr (kWide) // the CTA's code counts, added to its chunk's
     for (int i = threadIdx.x; i < int(kSeqHistWords); i += blockDim.x)
       if (shist[i]) {
         if (i == int(kSeqHistBad))
@@ -2103,9 +2104,15 @@ cudaError_t launch_zstd(CodecBatch b, void* scratch, cudaStream_t st)
       return e;
   }
   note_launches(4);
-  CHUCKY_LAUNCH(zstd_find_k, unsigned(b.n_chunks * rpc), 32 * kSegsPerRegion,
-                kRegionStageWords * sizeof(uint32_t), st, b, seqs, meta, hist, litbuf,
-                rpc, static_cast<const uint16_t*>(wide), seq_hist);
+  constexpr size_t smem = kRegionStageWords * sizeof(uint32_t);
+  const unsigned regions = unsigned(b.n_chunks * rpc);
+  if (wide)
+    CHUCKY_LAUNCH(zstd_find_k<true>, regions, 32 * kSegsPerRegion, smem, st, b, seqs, meta, hist,
+                  litbuf, rpc, static_cast<const uint16_t*>(wide), seq_hist);
+  else
+    CHUCKY_LAUNCH(zstd_find_k<false>, regions, 32 * kSegsPerRegion, smem, st, b, seqs, meta, hist,
+                  litbuf, rpc, static_cast<const uint16_t*>(nullptr),
+                  static_cast<uint32_t*>(nullptr));
   if ((e = cudaGetLastError()) != cudaSuccess)
     return e;
   static const PredefTables pre = [] {
