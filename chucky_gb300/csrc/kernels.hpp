@@ -68,9 +68,8 @@ cudaError_t launch_lod_emit(const LodMortonArgs& a,
                             const uint8_t* accum,
                             uint8_t* values,
                             cudaStream_t st);
-// (`levels`: a bit per level)
 cudaError_t launch_lod_to_chunks(const LodMortonArgs& a,
-                                 uint32_t levels,
+                                 int level,
                                  const uint8_t* values,
                                  uint8_t* slot,
                                  cudaStream_t st);

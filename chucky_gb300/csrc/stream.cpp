@@ -203,23 +203,14 @@ int Stream::setup_transpose()
   const tile_stream_layout& L = layout;
   const int r = L.lifted_rank;
   const uint64_t cs = L.lifted_shape[r - 1];
-  // A row of the tables: the innermost (count, chunk) pair, and pairs above
-  // it while the row stays below 1024 elements (3 channels: a row entry per 3
-  // elements would be read from memory with them) and the columns' table is
-  // one that the L1 and L2 hold.
-  int t = r - 2;
-  uint64_t width = L.lifted_shape[t] * cs;
-  while (t >= 2 && width < 1024 &&
-         width * L.lifted_shape[t - 2] * L.lifted_shape[t - 1] <= (1u << 16)) {
-    t -= 2;
-    width *= L.lifted_shape[t] * L.lifted_shape[t + 1];
-  }
+  const uint64_t width = L.lifted_shape[r - 2] * cs;
   const uint64_t rows = L.epoch_elements / width;
   std::vector<uint64_t> row(rows), col(width);
   for (uint64_t x = 0; x < width; ++x)
-    col[x] = ravel(r - t, L.lifted_shape + t, L.lifted_strides + t, x);
+    col[x] = (x / cs) * uint64_t(L.lifted_strides[r - 2]) +
+             (x % cs) * uint64_t(L.lifted_strides[r - 1]);
   for (uint64_t y = 0; y < rows; ++y)
-    row[y] = ravel(t, L.lifted_shape, L.lifted_strides, y);
+    row[y] = ravel(r - 2, L.lifted_shape, L.lifted_strides, y);
   CK(cudaMalloc(&d_row_off, rows * sizeof(uint64_t)));
   CK(cudaMalloc(&d_col_off, width * sizeof(uint64_t)));
   CK(cudaMemcpy(d_row_off, row.data(), rows * 8, cudaMemcpyHostToDevice));
@@ -706,7 +697,9 @@ int Stream::run_epoch(uint64_t present)
     }
     if (timed_begin(s_comp, &metrics.lod_morton_chunk, 0, double(P.slot_bytes)))
       return 1;
-    CK(launch_lod_to_chunks(lod, mask, d_values, slot_ptr, s_comp));
+    for (int l = 0; l < P.nlod; ++l)
+      if (mask >> l & 1)
+        CK(launch_lod_to_chunks(lod, l, d_values, slot_ptr, s_comp));
     if (timed_end(s_comp))
       return 1;
   }
@@ -1289,7 +1282,6 @@ writer_result Stream::append_async(slice in, cudaStream_t producer)
   const uint8_t* end = static_cast<const uint8_t*>(in.end);
   if (src >= end)
     return writer_result{ 0, { src, end } };
-  idle = false;
   const uint64_t ee = layout.epoch_elements;
   const double t0 = now_ms();
   const Source kind = classify(src, uint64_t(end - src), stage_small);
@@ -1392,7 +1384,7 @@ int Stream::flush_all()
           CK(launch_lod_drain(t, l, counts[l], s_comp));
         } else {
           CK(launch_lod_emit(lod, l, counts[l], d_accum, d_values, s_comp));
-          CK(launch_lod_to_chunks(lod, 1u << l, d_values, pool_slot(0), s_comp));
+          CK(launch_lod_to_chunks(lod, l, d_values, pool_slot(0), s_comp));
         }
         counts[l] = 0;
         drain |= 1u << l;
@@ -1427,7 +1419,6 @@ int Stream::flush_all()
     }
   }
   resolve_timers(true);
-  idle = true;
   return 0;
 }
 
@@ -1560,16 +1551,11 @@ tile_stream_gpu_restart(tile_stream_gpu* s, shard_sink* sink)
   Stream& I = s->impl;
   if (I.cursor != 0 && !I.flushed)
     return 1;
-  // After a flush that succeeded the host has waited for every batch, and
-  // the index kernel has left the index and cursors as they are at the start
-  // (it resets them with every shard epoch it completes): nothing to wait
-  // for or to clear.
-  const bool clean = I.idle;
-  if (!clean && (cudaStreamSynchronize(I.s_comp) != cudaSuccess ||
-                 cudaStreamSynchronize(I.s_enc[0]) != cudaSuccess ||
-                 cudaStreamSynchronize(I.s_enc[1]) != cudaSuccess ||
-                 cudaStreamSynchronize(I.s_agg) != cudaSuccess ||
-                 cudaStreamSynchronize(I.s_copy) != cudaSuccess))
+  if (cudaStreamSynchronize(I.s_comp) != cudaSuccess ||
+      cudaStreamSynchronize(I.s_enc[0]) != cudaSuccess ||
+      cudaStreamSynchronize(I.s_enc[1]) != cudaSuccess ||
+      cudaStreamSynchronize(I.s_agg) != cudaSuccess ||
+      cudaStreamSynchronize(I.s_copy) != cudaSuccess)
     return 1;
   if (sink)
     I.sink = sink;
@@ -1593,15 +1579,14 @@ tile_stream_gpu_restart(tile_stream_gpu* s, shard_sink* sink)
       sh.w = nullptr;
     }
     const uint64_t ns = I.P.lv[l].shard_inner_count;
-    if (!clean &&
-        (cudaMemsetAsync(I.d_index[l], 0xFF, ns * I.P.lv[l].cps_total * 16, I.s_comp) !=
-           cudaSuccess ||
-         cudaMemsetAsync(I.d_cursor[l], 0, ns * 8, I.s_comp) != cudaSuccess))
+    if (cudaMemsetAsync(I.d_index[l], 0xFF, ns * I.P.lv[l].cps_total * 16, I.s_comp) !=
+          cudaSuccess ||
+        cudaMemsetAsync(I.d_cursor[l], 0, ns * 8, I.s_comp) != cudaSuccess)
       return 1;
     I.kick_eis[l] = 0;
     I.io_done[l] = io_event{};
   }
-  if (!clean && cudaStreamSynchronize(I.s_comp) != cudaSuccess)
+  if (cudaStreamSynchronize(I.s_comp) != cudaSuccess)
     return 1;
   for (auto& sl : I.slot) {
     sl.busy = 0;
