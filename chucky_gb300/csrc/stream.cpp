@@ -203,14 +203,23 @@ int Stream::setup_transpose()
   const tile_stream_layout& L = layout;
   const int r = L.lifted_rank;
   const uint64_t cs = L.lifted_shape[r - 1];
-  const uint64_t width = L.lifted_shape[r - 2] * cs;
+  // A row of the tables: the innermost (count, chunk) pair, and pairs above
+  // it while the row stays below 1024 elements (3 channels: a row entry per 3
+  // elements would be read from memory with them) and the columns' table is
+  // one that the L1 and L2 hold.
+  int t = r - 2;
+  uint64_t width = L.lifted_shape[t] * cs;
+  while (t >= 2 && width < 1024 &&
+         width * L.lifted_shape[t - 2] * L.lifted_shape[t - 1] <= (1u << 16)) {
+    t -= 2;
+    width *= L.lifted_shape[t] * L.lifted_shape[t + 1];
+  }
   const uint64_t rows = L.epoch_elements / width;
   std::vector<uint64_t> row(rows), col(width);
   for (uint64_t x = 0; x < width; ++x)
-    col[x] = (x / cs) * uint64_t(L.lifted_strides[r - 2]) +
-             (x % cs) * uint64_t(L.lifted_strides[r - 1]);
+    col[x] = ravel(r - t, L.lifted_shape + t, L.lifted_strides + t, x);
   for (uint64_t y = 0; y < rows; ++y)
-    row[y] = ravel(r - 2, L.lifted_shape, L.lifted_strides, y);
+    row[y] = ravel(t, L.lifted_shape, L.lifted_strides, y);
   CK(cudaMalloc(&d_row_off, rows * sizeof(uint64_t)));
   CK(cudaMalloc(&d_col_off, width * sizeof(uint64_t)));
   CK(cudaMemcpy(d_row_off, row.data(), rows * 8, cudaMemcpyHostToDevice));

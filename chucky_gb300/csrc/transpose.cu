@@ -5,7 +5,9 @@
 // as src/gpu/transpose.cu:85-137 and src/cpu/transpose.cpp:10-105 of the
 // reference.  The innermost lifted pair (count, chunk) spans one input row
 // of `width` elements, so dst(e) = row_off[e / width] + col_off[e % width]:
-// the two small tables replace the per-element unravel.  When the chunk
+// the two small tables replace the per-element unravel.  (Where that pair
+// is narrow -- few channels innermost -- a row takes in the pairs above it.)
+// When the chunk
 // extent of the innermost dim is a multiple of 16 bytes and that dim is
 // innermost in storage, every 16-byte input vector lands in one contiguous,
 // aligned run of its chunk row: one 16-byte load and one 16-byte store per
@@ -33,18 +35,39 @@ transpose_vec16_k(TransposeArgs a, uint64_t nvec)
   }
 }
 
+// Elements one by one, where vectors do not stay whole: kRun consecutive ones
+// per thread, read with one or two vector loads and one division.  Bound by
+// its stores (an element each): RGB frames into planar u8 chunks (12.4 MB
+// epochs) took 67 us with a division and two table look-ups per byte, a table
+// entry per three bytes among them.
+constexpr uint32_t kRun = 4;
 template<typename T>
 __global__ void __launch_bounds__(kThreads)
 transpose_scalar_k(TransposeArgs a, uint64_t first)
 {
+  struct alignas(sizeof(T) * kRun < 16 ? sizeof(T) * kRun : 16) Run
+  {
+    T v[kRun];
+  };
   const T* src = reinterpret_cast<const T*>(a.src);
   T* dst = reinterpret_cast<T*>(a.dst);
-  for (uint64_t e = first + blockIdx.x * uint64_t(kThreads) + threadIdx.x;
-       e < a.n;
-       e += uint64_t(gridDim.x) * kThreads) {
+  // (`first` keeps the 16-byte alignment of the epoch buffer, which is padded)
+  for (uint64_t e = first + kRun * (blockIdx.x * uint64_t(kThreads) + threadIdx.x); e < a.n;
+       e += kRun * uint64_t(gridDim.x) * kThreads) {
+    const Run run = *reinterpret_cast<const Run*>(src + e);
     uint64_t row, x;
     a.width.divmod(e, row, x);
-    dst[__ldg(a.row_off + row) + __ldg(a.col_off + x)] = src[e];
+    uint64_t o = __ldg(a.row_off + row);
+#pragma unroll
+    for (uint32_t u = 0; u < kRun; ++u) {
+      if (e + u >= a.n)
+        break;
+      dst[o + __ldg(a.col_off + x)] = run.v[u];
+      if (++x == a.width.d && e + u + 1 < a.n) {
+        x = 0;
+        o = __ldg(a.row_off + ++row);
+      }
+    }
   }
 }
 
@@ -73,7 +96,7 @@ cudaError_t launch_transpose(const TransposeArgs& a, cudaStream_t st)
     }
   }
   if (first < a.n) {
-    const int g = grid_for(a.n - first);
+    const int g = grid_for((a.n - first + kRun - 1) / kRun);
     note_launches(1);
     switch (a.bpe) {
       case 1:
