@@ -68,8 +68,9 @@ cudaError_t launch_lod_emit(const LodMortonArgs& a,
                             const uint8_t* accum,
                             uint8_t* values,
                             cudaStream_t st);
+// (`levels`: a bit per level)
 cudaError_t launch_lod_to_chunks(const LodMortonArgs& a,
-                                 int level,
+                                 uint32_t levels,
                                  const uint8_t* values,
                                  uint8_t* slot,
                                  cudaStream_t st);

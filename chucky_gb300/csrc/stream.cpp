@@ -706,9 +706,7 @@ int Stream::run_epoch(uint64_t present)
     }
     if (timed_begin(s_comp, &metrics.lod_morton_chunk, 0, double(P.slot_bytes)))
       return 1;
-    for (int l = 0; l < P.nlod; ++l)
-      if (mask >> l & 1)
-        CK(launch_lod_to_chunks(lod, l, d_values, slot_ptr, s_comp));
+    CK(launch_lod_to_chunks(lod, mask, d_values, slot_ptr, s_comp));
     if (timed_end(s_comp))
       return 1;
   }
@@ -1393,7 +1391,7 @@ int Stream::flush_all()
           CK(launch_lod_drain(t, l, counts[l], s_comp));
         } else {
           CK(launch_lod_emit(lod, l, counts[l], d_accum, d_values, s_comp));
-          CK(launch_lod_to_chunks(lod, l, d_values, pool_slot(0), s_comp));
+          CK(launch_lod_to_chunks(lod, 1u << l, d_values, pool_slot(0), s_comp));
         }
         counts[l] = 0;
         drain |= 1u << l;
