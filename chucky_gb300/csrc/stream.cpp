@@ -1289,6 +1289,7 @@ writer_result Stream::append_async(slice in, cudaStream_t producer)
   const uint8_t* end = static_cast<const uint8_t*>(in.end);
   if (src >= end)
     return writer_result{ 0, { src, end } };
+  idle = false;
   const uint64_t ee = layout.epoch_elements;
   const double t0 = now_ms();
   const Source kind = classify(src, uint64_t(end - src), stage_small);
@@ -1426,6 +1427,7 @@ int Stream::flush_all()
     }
   }
   resolve_timers(true);
+  idle = true;
   return 0;
 }
 
@@ -1558,11 +1560,16 @@ tile_stream_gpu_restart(tile_stream_gpu* s, shard_sink* sink)
   Stream& I = s->impl;
   if (I.cursor != 0 && !I.flushed)
     return 1;
-  if (cudaStreamSynchronize(I.s_comp) != cudaSuccess ||
-      cudaStreamSynchronize(I.s_enc[0]) != cudaSuccess ||
-      cudaStreamSynchronize(I.s_enc[1]) != cudaSuccess ||
-      cudaStreamSynchronize(I.s_agg) != cudaSuccess ||
-      cudaStreamSynchronize(I.s_copy) != cudaSuccess)
+  // After a flush that succeeded the host has waited for every batch, and
+  // the index kernel has left the index and cursors as they are at the start
+  // (it resets them with every shard epoch it completes): nothing to wait
+  // for or to clear.
+  const bool clean = I.idle;
+  if (!clean && (cudaStreamSynchronize(I.s_comp) != cudaSuccess ||
+                 cudaStreamSynchronize(I.s_enc[0]) != cudaSuccess ||
+                 cudaStreamSynchronize(I.s_enc[1]) != cudaSuccess ||
+                 cudaStreamSynchronize(I.s_agg) != cudaSuccess ||
+                 cudaStreamSynchronize(I.s_copy) != cudaSuccess))
     return 1;
   if (sink)
     I.sink = sink;
@@ -1586,14 +1593,15 @@ tile_stream_gpu_restart(tile_stream_gpu* s, shard_sink* sink)
       sh.w = nullptr;
     }
     const uint64_t ns = I.P.lv[l].shard_inner_count;
-    if (cudaMemsetAsync(I.d_index[l], 0xFF, ns * I.P.lv[l].cps_total * 16, I.s_comp) !=
-          cudaSuccess ||
-        cudaMemsetAsync(I.d_cursor[l], 0, ns * 8, I.s_comp) != cudaSuccess)
+    if (!clean &&
+        (cudaMemsetAsync(I.d_index[l], 0xFF, ns * I.P.lv[l].cps_total * 16, I.s_comp) !=
+           cudaSuccess ||
+         cudaMemsetAsync(I.d_cursor[l], 0, ns * 8, I.s_comp) != cudaSuccess))
       return 1;
     I.kick_eis[l] = 0;
     I.io_done[l] = io_event{};
   }
-  if (cudaStreamSynchronize(I.s_comp) != cudaSuccess)
+  if (!clean && cudaStreamSynchronize(I.s_comp) != cudaSuccess)
     return 1;
   for (auto& sl : I.slot) {
     sl.busy = 0;

@@ -191,6 +191,7 @@ struct Stream
   uint32_t accumulated = 0;
   uint32_t masks[MAX_BATCH_EPOCHS] = {};
   int flushed = 0;
+  bool idle = false; // flushed with success, nothing appended since
 
   // metrics: event pairs resolved lazily
   struct Timer
