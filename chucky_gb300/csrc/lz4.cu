@@ -63,7 +63,7 @@ __host__ __device__ inline bool lz4_wide(int level) { return level >= 2; }
 // wide window (a kernel of their own: its registers would cost the other
 // levels a quarter of their warps).
 template<bool kWide>
-__global__ void __launch_bounds__(32 * kSegsPerRegion, kWide ? kWideCtas : 1)
+__global__ void __launch_bounds__(32 * kSegsPerRegion, kWide ? kWideCtas : kFindCtas)
 lz4_find_k(CodecBatch b,
            Seq* seqs,
            SegMeta* meta,

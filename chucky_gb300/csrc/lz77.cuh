@@ -96,6 +96,10 @@ __host__ __device__ constexpr uint64_t wide_entries(int hlog) { return uint64_t(
 // take 2.08 ms with 7 CTAs (60 KB of L1 left) and 3.3-3.6 ms with 8 or 9 (28
 // KB), 64 cube chunks at zstd level 3 1.79 ms with 7, 2.36 ms with 8.
 constexpr int kWideCtas = 7;
+// ... and the parse without it: as many as the shared memory of a region and
+// its tables allows (left alone, the zstd kernel took 92 registers: 1.20 ms
+// for 64 sensor chunks against 1.07)
+constexpr int kFindCtas = 9;
 // lanes whose local match is shorter than this probe the wide window
 constexpr uint32_t kWideProbeBelow = 16;
 
@@ -173,26 +177,37 @@ __device__ __forceinline__ void lz77_stage_region(const uint8_t* base,
 }
 
 // Length of the match of position q against cand (< q), up to kLaneExtend
-// bytes, ending at or before `end` (one lane).
+// bytes, ending at or before `end` (one lane).  The parse is bound by the
+// instructions it issues (85 % of the slots): with each staged word loaded
+// once here, one shuffle less per period and two instructions less per
+// chosen match below, the LZ4 finder went from 2.00 to 1.88 ms on 64 sensor
+// chunks.
 __device__ __forceinline__ uint32_t lane_match(const uint32_t* words,
                                                const uint8_t* bytes,
                                                uint32_t q,
                                                uint32_t cand,
                                                uint32_t end)
 {
-  uint32_t len = 4;
+  // 4 bytes per step, each staged word loaded once
+  const uint32_t sq = (q & 3) * 8, sc = (cand & 3) * 8;
+  const uint32_t* wq = words + (q >> 2) + 1;
+  const uint32_t* wc = words + (cand >> 2) + 1;
+  uint32_t q0 = wq[0], c0 = wc[0], len = 4;
   while (len < kLaneExtend) {
     if (q + len + 4 > end) { // the last bytes before `end`, one by one
       while (q + len < end && bytes[q + len] == bytes[cand + len])
         ++len;
       break;
     }
-    const uint32_t x = word_at(words, q + len) ^ word_at(words, cand + len);
+    const uint32_t q1 = *++wq, c1 = *++wc;
+    const uint32_t x = __funnelshift_r(q0, q1, sq) ^ __funnelshift_r(c0, c1, sc);
     if (x) {
       len += uint32_t(__ffs(int(x)) - 1) >> 3;
       break;
     }
     len += 4;
+    q0 = q1;
+    c0 = c1;
   }
   return len;
 }
@@ -404,8 +419,8 @@ __device__ __forceinline__ SegInfo lz77_parse_segment(const uint32_t* words,
       const uint32_t d = x > base ? x - base : 0;
       return step == 1 ? d : (d + step - 1) / step;
     };
-    int nxt = 32; // next hit lane after this lane's match
-    if ((hits >> lane) & 1) {
+    int nxt = 32; // next hit lane after this lane's match (a long one ends the chain)
+    if ((hits >> lane) & 1 && len < kLaneExtend) {
       const uint32_t f = lane_from(end_l);
       const unsigned nm = f >= 32 ? 0u : hits & (0xffffffffu << f);
       nxt = nm ? __ffs(int(nm)) - 1 : 32;
@@ -418,17 +433,12 @@ __device__ __forceinline__ SegInfo lz77_parse_segment(const uint32_t* words,
       if (!m)
         break;
       unsigned sel = 0;
-      int k = __ffs(int(m)) - 1, last = k;
-      for (;;) {
+      int k = __ffs(int(m)) - 1, last;
+      do {
         sel |= 1u << k;
         last = k;
-        if ((longs >> k) & 1)
-          break;
-        const int nk = __shfl_sync(0xffffffffu, nxt, k);
-        if (nk >= 32)
-          break;
-        k = nk;
-      }
+        k = __shfl_sync(0xffffffffu, nxt, k);
+      } while (k < 32);
       // the literals before a chosen match start at the previous chosen
       // match's end (the parse point for the first)
       const unsigned prev = sel & below_me;
@@ -500,9 +510,9 @@ __device__ __forceinline__ SegInfo lz77_parse_segment(const uint32_t* words,
     for (int i = 0; i < 3; ++i) {
       const uint32_t d = 1u << i;
       const uint32_t pa = __shfl_up_sync(0xffffffffu, xa, d);
-      const uint32_t pb0 = __shfl_up_sync(0xffffffffu, xb, d);
-      const uint32_t pb1 = __shfl_sync(0xffffffffu, xa, (lane + 32 - d) & 31);
-      const uint32_t pb = uint32_t(lane) >= d ? pb0 : pb1;
+      // (b's first lanes look back into a: a's last lanes hand on a's words)
+      const uint32_t pb =
+        __shfl_sync(0xffffffffu, uint32_t(lane) >= 32 - d ? xa : xb, (lane + 32 - d) & 31);
       if (va && !oka && uint32_t(lane) >= d && pa == xa) {
         ca = qa - d * step;
         oka = true;

@@ -214,7 +214,7 @@ constexpr uint32_t kSeqHistWords = 128;
 
 // (kWide as in lz4_find_k.)
 template<bool kWide>
-__global__ void __launch_bounds__(32 * kSegsPerRegion, kWide ? kWideCtas : 1)
+__global__ void __launch_bounds__(32 * kSegsPerRegion, kWide ? kWideCtas : kFindCtas)
 zstd_find_k(CodecBatch b,
             Seq* seqs,
             ZSeg* meta,
