@@ -1510,15 +1510,30 @@ zstd_block_k(CodecBatch b,
   const ChunkTable& ct = tables[chunk];
   for (int c = tid; c < 256; c += blockDim.x)
     S.cl[c] = ct.cl[c];
+  // Most blocks of noisy data have no sequences: no tables for them, and no
+  // barriers of the sequences section below.
+  uint32_t nseq_all = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kSegsPerBlock; ++k)
+    if (k < nsegs)
+      nseq_all += meta[segbase + k].nseq;
   // the three sequence tables: the chunk's (adaptive) or the predefined
   // ones (built once on the host)
-  {
+  if (nseq_all) {
     static_assert(sizeof(PredefTables) == 3 * sizeof(SeqEnc), "LL, ML, OF in a row");
     const uint32_t* src = cseq ? reinterpret_cast<const uint32_t*>(cseq[chunk].t)
                                : reinterpret_cast<const uint32_t*>(&pre);
     uint32_t* dst = reinterpret_cast<uint32_t*>(&S.seqt);
     for (int i = tid; i < int(sizeof(PredefTables) / 4); i += blockDim.x)
       dst[i] = src[i];
+    for (int i = tid; i < 53; i += blockDim.x) {
+      S.ml_base[i] = kMLBase[i];
+      S.ml_bits[i] = kMLBits[i];
+      if (i < 36) {
+        S.ll_base[i] = kLLBase[i];
+        S.ll_bits[i] = kLLBits[i];
+      }
+    }
   }
   if (tid == 0) {
     // modes byte (LL, OF, ML in bits 7-6, 5-4, 3-2): a described table is
@@ -1535,14 +1550,6 @@ zstd_block_k(CodecBatch b,
     }
     S.seq_modes = modes;
     S.seq_desc = desc;
-  }
-  for (int i = tid; i < 53; i += blockDim.x) {
-    S.ml_base[i] = kMLBase[i];
-    S.ml_bits[i] = kMLBits[i];
-    if (i < 36) {
-      S.ll_base[i] = kLLBase[i];
-      S.ll_bits[i] = kLLBits[i];
-    }
   }
   if (tid == 0) {
     // the block's segment records, loaded together
@@ -1590,6 +1597,24 @@ zstd_block_k(CodecBatch b,
     S.lit_same = lit_same;
     S.lit_missing = 0;
     S.seq_bad = 0;
+    // literals section mode (the exact Huffman size decides below).  In a
+    // treeless chunk the carrier block describes the table and is always
+    // kept as a compressed block; later blocks refer to its description.
+    S.lit_mode = 0;
+    S.with_desc = 1;
+    S.forced = 0;
+    if (S.nlit > 0 && lit_same)
+      S.lit_mode = 1;
+    else if (block_uses_table(ct.ok, S.nlit, false)) {
+      S.lit_mode = 2;
+      if (ct.carrier != ~0u) {
+        S.with_desc = bi == ct.carrier;
+        S.forced = bi == ct.carrier;
+      }
+    }
+    // the block describing the chunk's sequence tables stays compressed too
+    if (S.seq_desc)
+      S.forced = 1;
   }
   __syncthreads();
 
@@ -1602,27 +1627,6 @@ zstd_block_k(CodecBatch b,
   }
   __syncthreads();
   const uint32_t nlit = S.nlit, nseq = S.nseq;
-  if (tid == 0) {
-    // literals section mode (the exact Huffman size decides below).  In a
-    // treeless chunk the carrier block describes the table and is always
-    // kept as a compressed block; later blocks refer to its description.
-    S.lit_mode = 0;
-    S.with_desc = 1;
-    S.forced = 0;
-    if (nlit > 0 && S.lit_same)
-      S.lit_mode = 1;
-    else if (block_uses_table(ct.ok, nlit, false)) {
-      S.lit_mode = 2;
-      if (ct.carrier != ~0u) {
-        S.with_desc = bi == ct.carrier;
-        S.forced = bi == ct.carrier;
-      }
-    }
-    // the block describing the chunk's sequence tables stays compressed too
-    if (S.seq_desc)
-      S.forced = 1;
-  }
-  __syncthreads();
 
   // ---- Huffman streams: bit lengths per stream (64 threads per stream)
   const uint32_t per = (nlit + 3) / 4;
@@ -1836,57 +1840,71 @@ zstd_block_k(CodecBatch b,
   // on all threads.  The literal buffer is free again (the literals are in
   // staging) and holds the per-sequence codes, then the states.
   uint8_t* scode = lits; // [3][nseq]: LL, ML, OF codes -> states (in place)
-  for (uint32_t j = tid; j < nseq; j += blockDim.x) {
-    uint32_t ll, ml, off;
-    seq_at(S, seqs, segbase, nsegs, j, ll, ml, off);
-    const int oc = highbit(off);
-    if (oc > 28 || ml < 3 || off <= 3)
-      S.seq_bad = 1;
-    scode[j] = uint8_t(ll_code(ll));
-    scode[nseq + j] = uint8_t(ml < 3 ? 0 : ml_code(ml));
-    scode[2 * nseq + j] = uint8_t(oc);
-  }
-  __syncthreads();
-  if (warp == 0 && lane < 3 && nseq) {
-    const SeqEnc& t = lane == 0 ? S.seqt.ll : (lane == 1 ? S.seqt.ml : S.seqt.of);
-    uint8_t* a = scode + lane * nseq;
-    const uint32_t size = 1u << t.al;
-    uint32_t v = t.states[t.first[a[nseq - 1]]] + size;
-    for (int j = int(nseq) - 2; j >= 0; --j) {
-      const int sym = a[j];
-      a[j] = uint8_t(v - size);
-      const int c = t.count[sym];
-      int nb = t.al - highbit(uint32_t(c));
-      if ((v >> nb) < uint32_t(c))
-        --nb;
-      v = t.states[t.first[sym] + ((v >> nb) - c)] + size;
+  uint32_t p0 = 0, p1 = 0, before = 0, total_bits = 0;
+  if (nseq) { // (the whole CTA)
+    for (uint32_t j = tid; j < nseq; j += blockDim.x) {
+      uint32_t ll, ml, off;
+      seq_at(S, seqs, segbase, nsegs, j, ll, ml, off);
+      const int oc = highbit(off);
+      if (oc > 28 || ml < 3 || off <= 3)
+        S.seq_bad = 1;
+      scode[j] = uint8_t(ll_code(ll));
+      scode[nseq + j] = uint8_t(ml < 3 ? 0 : ml_code(ml));
+      scode[2 * nseq + j] = uint8_t(oc);
     }
-    S.final_state[lane] = v - size;
-  }
-  __syncthreads();
-  // sequence p of the stream is block sequence nseq - 1 - p (written
-  // backwards); thread tid packs the stream sequences [p0, p1)
-  const uint32_t p0 = uint32_t(uint64_t(nseq) * tid / kBlockThreads);
-  const uint32_t p1 = uint32_t(uint64_t(nseq) * (tid + 1) / kBlockThreads);
-  uint32_t my_bits = 0;
-  for (uint32_t p = p0; p < p1; ++p)
-    my_bits += seq_emit(S, seqs, segbase, nsegs, nseq, scode, nseq - 1 - p,
-                        [](uint32_t, int) {});
-  uint32_t before = my_bits;
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, before, o);
-    if (lane >= o)
-      before += y;
-  }
-  if (lane == 31)
-    S.warp_bits[warp] = before;
-  before -= my_bits;
-  __syncthreads();
-  uint32_t total_bits = 0;
-  for (int w = 0; w < kBlockThreads / 32; ++w) {
-    if (w < warp)
-      before += S.warp_bits[w];
-    total_bits += S.warp_bits[w];
+    __syncthreads();
+    if (warp == 0 && lane < 3) {
+      const SeqEnc& t = lane == 0 ? S.seqt.ll : (lane == 1 ? S.seqt.ml : S.seqt.of);
+      uint8_t* a = scode + lane * nseq;
+      const uint32_t size = 1u << t.al;
+      uint32_t v = t.states[t.first[a[nseq - 1]]] + size;
+      // A step waits for one load only, that of its state: the codes are read
+      // two steps ahead and their counts and first states one.
+      struct Code
+      {
+        int c, first, nb; // count, first state, bits when the state is large
+      };
+      auto look = [&](int sym) {
+        const int c = t.count[sym];
+        return Code{ c, int(t.first[sym]) - c, t.al - highbit(uint32_t(c)) };
+      };
+      int j = int(nseq) - 2;
+      int sym1 = a[j >= 1 ? j - 1 : int(nseq) - 1]; // (any code once there is none)
+      Code next = look(a[j >= 0 ? j : int(nseq) - 1]);
+      for (; j >= 0; --j) {
+        const Code k = next;
+        a[j] = uint8_t(v - size);
+        next = look(sym1);
+        sym1 = j >= 2 ? a[j - 2] : sym1;
+        const int nb = k.nb - ((v >> k.nb) < uint32_t(k.c) ? 1 : 0);
+        v = t.states[k.first + int(v >> nb)] + size;
+      }
+      S.final_state[lane] = v - size;
+    }
+    __syncthreads();
+    // sequence p of the stream is block sequence nseq - 1 - p (written
+    // backwards); thread tid packs the stream sequences [p0, p1)
+    p0 = uint32_t(uint64_t(nseq) * tid / kBlockThreads);
+    p1 = uint32_t(uint64_t(nseq) * (tid + 1) / kBlockThreads);
+    uint32_t my_bits = 0;
+    for (uint32_t p = p0; p < p1; ++p)
+      my_bits += seq_emit(S, seqs, segbase, nsegs, nseq, scode, nseq - 1 - p,
+                          [](uint32_t, int) {});
+    before = my_bits;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, before, o);
+      if (lane >= o)
+        before += y;
+    }
+    if (lane == 31)
+      S.warp_bits[warp] = before;
+    before -= my_bits;
+    __syncthreads();
+    for (int w = 0; w < kBlockThreads / 32; ++w) {
+      if (w < warp)
+        before += S.warp_bits[w];
+      total_bits += S.warp_bits[w];
+    }
   }
   // header: sequence count, then the modes byte and (carrier) the table
   // descriptions
@@ -1895,7 +1913,8 @@ zstd_block_k(CodecBatch b,
     nseq == 0 ? 1 : (nseq < 128 ? 2 : (nseq < 0x7F00 ? 3 : 4)) + S.seq_desc;
   const uint32_t bs0 = seq_at0 + nhdr; // first byte of the bitstream
   // final states and the end mark
-  const uint32_t fin_bits = uint32_t(S.seqt.ll.al + S.seqt.ml.al + S.seqt.of.al);
+  const uint32_t fin_bits =
+    nseq ? uint32_t(S.seqt.ll.al + S.seqt.ml.al + S.seqt.of.al) : 0;
   const uint32_t nbytes = nseq ? (total_bits + fin_bits + 1 + 7) / 8 : 0;
   const bool fits = bs0 + nbytes + 4 <= kStageBytes && !S.seq_bad;
   if (fits) {
