@@ -120,6 +120,7 @@ struct ChunkRuns
 // Scratch of one launch set.  The level selects the parse: LZ4 levels >= 2
 // and zstd levels >= 3 also search the wide window (earlier regions of the
 // chunk) and need room for its region tables.
+constexpr int kLz4WideLevel = 2, kZstdWideLevel = 3;
 size_t lz4_scratch_bytes(uint64_t n_chunks, uint32_t chunk_bytes, int level);
 cudaError_t launch_lz4(CodecBatch b, void* scratch, cudaStream_t st);
 

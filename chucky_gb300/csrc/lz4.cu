@@ -57,7 +57,7 @@ struct SegMeta
 // one, LZ4's 64 KiB reach); level 0 and 1 with the region's own window.
 constexpr uint32_t kLz4WideBack = 3;
 constexpr int kLz4WideLog = 15;
-__host__ __device__ inline bool lz4_wide(int level) { return level >= 2; }
+__host__ __device__ inline bool lz4_wide(int level) { return level >= kLz4WideLevel; }
 
 // One CTA per region, a warp per segment of it.  kWide: the levels with the
 // wide window (a kernel of their own: its registers would cost the other

@@ -73,6 +73,25 @@ double now_ms()
     .count();
 }
 
+// Whether a batch's encoders wait for those of the batch before it (the two
+// batches in flight have a stream each), so that the earlier batch's bytes
+// are on the link while the later one is encoded.  Side by side, both finish
+// late and their copies to the host queue up behind them.
+//
+// From 64 MiB of chunks a batch fills the chip by itself (a warp parses
+// 4 KiB: three waves of the 152 x 9 resident CTAs) and order costs nothing:
+// two batches of 302 MB sensor frames, zstd-1, 5.21 ms side by side and
+// 4.75 in order; of 67 MB, 1.31 and 1.26 (LZ4 2.24 and 2.15).  Below it
+// leaves SMs idle: 33.6 MB zstd-1 0.73 and 0.81 ms.  The wide window's parse
+// is a long serial chain per warp, whose last wave the other batch fills at
+// every size: 302 MB zstd-3 30.7 and 31.5 ms, 67 MB 7.1 and 7.7.
+constexpr uint64_t kEncodeInOrderBytes = 64ull << 20;
+bool encode_in_order(const tile_stream_configuration& cfg, uint64_t bytes)
+{
+  const int wide = cfg.codec.id == CODEC_ZSTD ? kZstdWideLevel : kLz4WideLevel;
+  return cfg.codec.level < wide && bytes >= kEncodeInOrderBytes;
+}
+
 } // namespace
 
 // ---------------------------------------------------------------------------
@@ -818,6 +837,8 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
         return 1;
       CK(cudaStreamWaitEvent(se, ev_engine_done[si], 0));
     } else {
+      if (encode_in_order(cfg, n * P.chunk_bytes))
+        CK(cudaStreamWaitEvent(se, ev_codec_done[si ^ 1], 0));
       if (timed_begin(se, &metrics.compress, double(n * P.chunk_bytes), 0))
         return 1;
       if (codec_compress(comp, n, d_ids, rp, d_comp[si], d_sizes[si], codec_state[si], se))

@@ -205,7 +205,7 @@ constexpr int kZstdWideLog = 14;
 #define CHUCKY_ZSTD_MIN_MATCH_WIDE 4
 #endif
 constexpr uint32_t kMinMatchWide = CHUCKY_ZSTD_MIN_MATCH_WIDE;
-__host__ __device__ inline bool zstd_wide(int level) { return level >= 3; }
+__host__ __device__ inline bool zstd_wide(int level) { return level >= kZstdWideLevel; }
 // Per-chunk counts of the sequence codes (levels with the wide window):
 // LL codes at 0, ML codes at kSeqHistML, OF codes at kSeqHistOF; a word
 // set when a sequence cannot be coded.
