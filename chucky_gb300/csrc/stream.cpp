@@ -1306,11 +1306,18 @@ writer_result Stream::append_async(slice in, cudaStream_t producer)
 {
   if (flushed)
     return writer_finished_at(in.beg, in.end);
+  idle = false;
+  const writer_result r = append_slice(in, producer);
+  failed |= r.error == writer_error_fail;
+  return r;
+}
+
+writer_result Stream::append_slice(slice in, cudaStream_t producer)
+{
   const uint8_t* src = static_cast<const uint8_t*>(in.beg);
   const uint8_t* end = static_cast<const uint8_t*>(in.end);
   if (src >= end)
     return writer_result{ 0, { src, end } };
-  idle = false;
   const uint64_t ee = layout.epoch_elements;
   const double t0 = now_ms();
   const Source kind = classify(src, uint64_t(end - src), stage_small);
@@ -1448,7 +1455,6 @@ int Stream::flush_all()
     }
   }
   resolve_timers(true);
-  idle = true;
   return 0;
 }
 
@@ -1458,6 +1464,8 @@ writer_result Stream::flush()
     return writer_finished_at(nullptr, nullptr);
   const int rc = flush_all();
   flushed = 1;
+  failed |= rc != 0;
+  idle = !failed;
   return rc ? writer_error() : writer_ok();
 }
 
@@ -1581,10 +1589,10 @@ tile_stream_gpu_restart(tile_stream_gpu* s, shard_sink* sink)
   Stream& I = s->impl;
   if (I.cursor != 0 && !I.flushed)
     return 1;
-  // After a flush that succeeded the host has waited for every batch, and
-  // the index kernel has left the index and cursors as they are at the start
-  // (it resets them with every shard epoch it completes): nothing to wait
-  // for or to clear.
+  // After appends and a flush that all succeeded the host has waited for
+  // every batch, and the index kernel has left the index and cursors as they
+  // are at the start (it resets them with every shard epoch it completes):
+  // nothing to wait for or to clear.
   const bool clean = I.idle;
   if (!clean && (cudaStreamSynchronize(I.s_comp) != cudaSuccess ||
                  cudaStreamSynchronize(I.s_enc[0]) != cudaSuccess ||
@@ -1596,6 +1604,7 @@ tile_stream_gpu_restart(tile_stream_gpu* s, shard_sink* sink)
     I.sink = sink;
   I.cursor = 0;
   I.flushed = 0;
+  I.failed = false;
   I.stage_fill = 0;
   for (bool& u : I.stage_used)
     u = false;

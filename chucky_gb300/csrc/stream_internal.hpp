@@ -191,7 +191,8 @@ struct Stream
   uint32_t accumulated = 0;
   uint32_t masks[MAX_BATCH_EPOCHS] = {};
   int flushed = 0;
-  bool idle = false; // flushed with success, nothing appended since
+  bool failed = false; // an append or the flush failed since the (re)start
+  bool idle = false;   // flushed, with no failure before, nothing appended since
 
   // metrics: event pairs resolved lazily
   struct Timer
@@ -233,6 +234,7 @@ struct Stream
   // of the caller): the copies wait for the producer's work so far, and the
   // producer's later work waits for the copies; the host does not wait.
   writer_result append_async(slice in, cudaStream_t producer);
+  writer_result append_slice(slice in, cudaStream_t producer);
   writer_result flush();
   int stage_issue();
   int stage_copy(uint8_t* dst, const uint8_t* src, uint64_t bytes);
