@@ -485,9 +485,8 @@ int Stream::setup_aggregate()
       DeliverySlot::Level& D = slot[s].lv[l];
       D.positions_cap = positions;
       D.data_cap = data;
-      CK(cudaHostAlloc(&D.offsets, (positions + 1) * 8, cudaHostAllocMapped));
-      CK(cudaMalloc(&D.d_offsets, (positions + 1) * 8));
-      CK(cudaMalloc(&D.real_sizes, positions * 8 + 8));
+      CK(cudaMalloc(&D.d_offsets, 2 * (positions + 1) * 8));
+      D.real_sizes = D.d_offsets + positions + 1;
       CK(cudaHostAlloc(&D.data, data, cudaHostAllocMapped));
       if (slots_on_device)
         CK(cudaMalloc(&D.d_data, data));
@@ -502,16 +501,25 @@ int Stream::setup_aggregate()
     CK(cudaMemset(d_index[l], 0xFF, V.shard_inner_count * nidx));
     CK(cudaMalloc(&d_cursor[l], V.shard_inner_count * 8));
     CK(cudaMemset(d_cursor[l], 0, V.shard_inner_count * 8));
-    CK(cudaHostAlloc(&h_flush_blobs[l], V.shard_inner_count * blob_bytes[l],
-                     cudaHostAllocMapped));
     const uint32_t finals = cap_epochs / uint32_t(std::max<uint64_t>(1, V.cps_append)) + 2;
+    // the level's small mapped blocks in one allocation, each from a page on
+    // (pinning takes the host about 0.2 ms a block)
+    const uint64_t page = 4096;
+    const uint64_t flush_n = round_up(V.shard_inner_count * blob_bytes[l], page);
+    const uint64_t offsets_n = round_up((positions + 1) * 8, page);
+    const uint64_t runs_n = round_up((cap_epochs + 2) * sizeof(IndexRun), page);
+    const uint64_t blobs_n = round_up(finals * V.shard_inner_count * blob_bytes[l], page);
+    CK(cudaHostAlloc(&h_flush_blobs[l], flush_n + 2 * (offsets_n + runs_n + blobs_n),
+                     cudaHostAllocMapped));
+    uint8_t* at = h_flush_blobs[l] + flush_n;
     for (int si = 0; si < 2; ++si) {
       DeliverySlot::Level& D = slot[si].lv[l];
       D.runs_cap = cap_epochs + 2;
       D.finals_cap = finals;
-      CK(cudaHostAlloc(&D.runs, D.runs_cap * sizeof(IndexRun), cudaHostAllocMapped));
-      CK(cudaHostAlloc(&D.blobs, finals * V.shard_inner_count * blob_bytes[l],
-                       cudaHostAllocMapped));
+      D.offsets = reinterpret_cast<uint64_t*>(at);
+      D.runs = reinterpret_cast<IndexRun*>(at + offsets_n);
+      D.blobs = at + offsets_n + runs_n;
+      at += offsets_n + runs_n + blobs_n;
     }
   }
   agg_scratch_slot = (max_positions + 1) * size_t(P.nlod);
@@ -552,11 +560,7 @@ void Stream::release()
     if (ev_batch[i])
       cudaEventDestroy(ev_batch[i]);
     for (int l = 0; l < LOD_MAX_LEVELS; ++l) {
-      cudaFreeHost(slot[i].lv[l].runs);
-      cudaFreeHost(slot[i].lv[l].blobs);
-      cudaFreeHost(slot[i].lv[l].offsets);
-      cudaFree(slot[i].lv[l].d_offsets);
-      cudaFree(slot[i].lv[l].real_sizes);
+      cudaFree(slot[i].lv[l].d_offsets); // (real_sizes with it)
       cudaFreeHost(slot[i].lv[l].data);
       cudaFree(slot[i].lv[l].d_data);
     }
@@ -598,7 +602,7 @@ void Stream::release()
   for (int l = 0; l < LOD_MAX_LEVELS; ++l) {
     cudaFree(d_index[l]);
     cudaFree(d_cursor[l]);
-    cudaFreeHost(h_flush_blobs[l]);
+    cudaFreeHost(h_flush_blobs[l]); // (the slots' offsets, runs and blobs with it)
     d_index[l] = d_cursor[l] = nullptr;
     h_flush_blobs[l] = nullptr;
     cudaFree(d_chunk_lut[l]);
