@@ -225,11 +225,11 @@ int Stream::setup_transpose()
   // A row of the tables: the innermost (count, chunk) pair, and pairs above
   // it while the row stays below 1024 elements (3 channels: a row entry per 3
   // elements would be read from memory with them) and the columns' table is
-  // one that the L1 and L2 hold.
+  // one that the L2 holds and the host makes in a moment.
   int t = r - 2;
   uint64_t width = L.lifted_shape[t] * cs;
   while (t >= 2 && width < 1024 &&
-         width * L.lifted_shape[t - 2] * L.lifted_shape[t - 1] <= (1u << 16)) {
+         width * L.lifted_shape[t - 2] * L.lifted_shape[t - 1] <= (1u << 14)) {
     t -= 2;
     width *= L.lifted_shape[t] * L.lifted_shape[t + 1];
   }
@@ -249,6 +249,19 @@ int Stream::setup_transpose()
   tr.bpe = uint32_t(P.bpe);
   tr.vector_ok = L.lifted_strides[r - 1] == 1 && (cs * P.bpe) % 16 == 0 &&
                  16 % P.bpe == 0;
+  // Interleaved channels: every 16 bytes' worth of pixels is 16 bytes of one
+  // chunk row in each channel.
+  const uint64_t channels = L.lifted_shape[r - 2] * cs;
+  bool planar = !tr.vector_ok && 16 % P.bpe == 0 && channels >= 2 && channels <= 4 && r >= 4 &&
+                L.lifted_strides[r - 3] == 1 && (L.lifted_shape[r - 3] * P.bpe) % 16 == 0;
+  for (int d = 0; d < r && planar; ++d)
+    planar = d == r - 3 || L.lifted_shape[d] == 1 ||
+             (uint64_t(L.lifted_strides[d]) * P.bpe) % 16 == 0;
+  if (planar) {
+    tr.channels = uint32_t(channels);
+    for (uint64_t c = 0; c < channels; ++c)
+      tr.channel_off[c] = ravel(2, L.lifted_shape + r - 2, L.lifted_strides + r - 2, c);
+  }
   return 0;
 }
 
