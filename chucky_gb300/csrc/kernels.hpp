@@ -136,11 +136,6 @@ struct AggBatch
   AggLevel lv[32];
 };
 
-// sizes -> shard order -> page pad -> exclusive scan, then gather bytes.
-cudaError_t launch_aggregate(const AggBatch& b,
-                             uint64_t* scratch, // >= max positions
-                             cudaStream_t st);
-
 // Shard index (src/zarr/shard_delivery.c:36-102), built on the device.
 // Per level the index of every shard of the current shard epoch
 // (cps_total (offset, nbytes) u64 pairs, all ones for an empty slot) and
@@ -180,6 +175,13 @@ struct IndexBatch
   IndexLevel lv[32];
 };
 cudaError_t launch_index(const IndexBatch& b, cudaStream_t st);
+
+// sizes -> shard order -> page pad -> exclusive scan, then gather bytes and,
+// if given, build the index of the same batch beside the gather.
+cudaError_t launch_aggregate(const AggBatch& b,
+                             uint64_t* scratch,       // >= max positions
+                             const IndexBatch* index, // or null
+                             cudaStream_t st);
 
 // The rest of a batch's shard-ordered bytes after a copy-engine transfer of
 // the expected size: per level, bytes [start, *total) of `src` (device) to
