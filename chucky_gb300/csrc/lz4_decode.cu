@@ -22,10 +22,14 @@
 // A sequence that does not fit a tile or whose length bytes run on (long
 // literal runs, long matches) is copied by the whole CTA.
 //
+// With few blocks two CTAs work on each, one parsing and placing ahead of the
+// other's execution (lz4_decode_pair_k).
+//
 // Bound by the integer instructions of the parse and of the tiles (about 20
 // us for a 16 KiB tile: 5 chain steps, 2 chain, 5 sequences, 8 tile), not by
-// memory: 64 sensor chunks of 1 MiB take 1.39 ms (a warp per block, sequence
-// by sequence: 62.3 ms), 1,024 of 16 KiB 0.15 ms.
+// memory: 64 sensor chunks of 1 MiB take 1.00 ms with two CTAs each, 1.39
+// with one (a warp per block, sequence by sequence: 62.3 ms), 1,024 of 16 KiB
+// 0.15 ms.
 //
 // Every read is checked against the block's size and every write against
 // the chunk size.  A block the fast path cannot finish is decoded once more
@@ -267,7 +271,23 @@ __device__ bool lz4_long_length(LzShared<NT>& S,
   return true;
 }
 
-// One sequence of any length at ip, by the whole CTA; false: malformed.
+// What the parse hands to the execution: a tile whose sequences are listed
+// (lit: its bytes), or one sequence of any length.
+struct LzWork
+{
+  enum : uint32_t
+  {
+    kDone,
+    kTile,
+    kLong,
+  };
+  uint32_t kind;
+  const uint8_t* lits; // (a tile: the window's first byte)
+  uint8_t* to;
+  uint64_t lit, off, ml;
+};
+
+// One sequence of any length at ip, read by the whole CTA; false: malformed.
 template<int NT>
 __device__ bool lz4_long_sequence(LzShared<NT>& S,
                                   const uint8_t* src,
@@ -276,9 +296,9 @@ __device__ bool lz4_long_sequence(LzShared<NT>& S,
                                   uint64_t chunk_bytes,
                                   uint64_t& ip,
                                   uint64_t& op,
-                                  bool& last)
+                                  bool& last,
+                                  LzWork& q)
 {
-  const unsigned tid = threadIdx.x;
   if (ip >= n)
     return false;
   const uint32_t token = src[ip++];
@@ -287,7 +307,7 @@ __device__ bool lz4_long_sequence(LzShared<NT>& S,
     return false;
   if (lit > n - ip || lit > chunk_bytes - op)
     return false;
-  copy_exact(dst + op, src + ip, lit, tid, NT);
+  q = LzWork{ LzWork::kLong, src + ip, dst + op, lit, 0, 0 };
   ip += lit;
   op += lit;
   last = ip == n;
@@ -295,23 +315,47 @@ __device__ bool lz4_long_sequence(LzShared<NT>& S,
     return true;
   if (n - ip < 2)
     return false;
-  const uint64_t off = uint64_t(src[ip]) | uint64_t(src[ip + 1]) << 8;
+  q.off = uint64_t(src[ip]) | uint64_t(src[ip + 1]) << 8;
   ip += 2;
-  uint64_t ml = (token & 15) + 4;
-  if (ml == 19 && !lz4_long_length(S, src, n, ip, ml))
+  q.ml = (token & 15) + 4;
+  if (q.ml == 19 && !lz4_long_length(S, src, n, ip, q.ml))
     return false;
-  if (off == 0 || off > op || ml > chunk_bytes - op)
+  if (q.off == 0 || q.off > op || q.ml > chunk_bytes - op)
     return false;
-  __syncthreads(); // the literals
-  cta_match<NT>(dst + op, off, ml);
-  op += ml;
-  __syncthreads();
+  op += q.ml;
   return true;
 }
 
-// `n` bytes of a block at src by all NT threads; false when it is malformed.
+// ... and copied by the whole CTA
 template<int NT>
+__device__ void lz4_copy_long(const LzWork& q)
+{
+  copy_exact(q.to, q.lits, q.lit, threadIdx.x, NT);
+  __syncthreads(); // the literals
+  if (q.ml)
+    cta_match<NT>(q.to + q.lit, q.off, q.ml);
+  __syncthreads();
+}
+
+// A CTA executes what it has parsed: the list is in its shared memory.
+template<int NT>
+struct LzOwn
+{
+  LzShared<NT>& S;
+  __device__ LzTok* tok() { return S.t.tok; }
+  __device__ void tile(const uint8_t*, const uint8_t* b, uint8_t* to, uint32_t nout)
+  {
+    // (a last sequence of no bytes follows all marked ones)
+    tile_run<NT, 6>(S.t.tile, S.warp_sum, S.t.tok, b, to, nout);
+  }
+  __device__ void run_long(const LzWork& q) { lz4_copy_long<NT>(q); }
+};
+
+// `n` bytes of a block at src by all NT threads; false when it is malformed.
+// X: who executes the tiles.
+template<int NT, typename X>
 __device__ bool lz4_decode_tiles(LzShared<NT>& S,
+                                 X& exec,
                                  const uint8_t* src,
                                  const uint64_t n,
                                  uint8_t* dst,
@@ -446,8 +490,8 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
           S.cut_out = out;
         }
         if (out + len <= LzTile<NT>::kBytes) {
-          S.t.tok[k + 1].bound = uint16_t(shd + out + l);
-          S.t.tok[k + 1].dlit = int32_t(a) - int32_t(shd + out);
+          exec.tok()[k + 1] =
+            LzTok{ uint16_t(shd + out + l), t.off, int32_t(a) - int32_t(shd + out) };
           if (t.off > op + out + l)
             S.bad = 1;
           if (len)
@@ -468,15 +512,17 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
         return false;
       if (used == 0) { // a sequence that fits neither window nor tile
         bool last = false;
-        if (!lz4_long_sequence(S, src, n, dst, chunk_bytes, ip, op, last))
+        LzWork q;
+        __syncthreads(); // (S.bad and S.cut have been read)
+        if (!lz4_long_sequence(S, src, n, dst, chunk_bytes, ip, op, last, q))
           return false;
+        exec.run_long(q);
         if (last)
           return op == chunk_bytes;
         want = Sh::kWindow;
         continue;
       }
-      // (a last sequence of no bytes follows all marked ones)
-      tile_run<NT, 6>(S.t.tile, S.warp_sum, S.t.tok, b, dst + op, nout);
+      exec.tile(src + ip, b, dst + op, nout);
       ip += used;
       op += nout;
       if (!cut && chain_end == kEnd)
@@ -507,7 +553,8 @@ lz4_decode_k(const uint8_t* in,
     const uint8_t* src = in + in_off[c];
     const uint64_t n = in_size[c];
     uint8_t* dst = out + c * out_stride;
-    const bool ok = lz4_decode_tiles<NT>(S, src, n, dst, chunk_bytes);
+    LzOwn<NT> own{ S };
+    const bool ok = lz4_decode_tiles<NT>(S, own, src, n, dst, chunk_bytes);
     __syncthreads();
     if (threadIdx.x < 32) {
       const uint32_t st =
@@ -518,6 +565,138 @@ lz4_decode_k(const uint8_t* in,
     __syncthreads();
   }
 }
+
+#ifndef CHUCKY_LZ4_UNPAIRED // (the CPU emulation of the kernels has no clusters)
+// Two CTAs per block, a cluster: the first parses the block and lists the
+// sequences of one tile after another in the second's shared memory, the
+// second executes a tile while the first parses the next.  A cluster barrier
+// per tile; both CTAs pass the same ones: the first ends its block with a
+// kDone of its own, the second leaves its loop only there.  Bound by the parse
+// and placement (12 of 20 us per tile), the longer half.
+template<int NT>
+struct LzPairShared // the second CTA's
+{
+  LzTile<NT> tile;
+  struct
+  {
+    LzWork work;
+    uint32_t start[NT / 2 + 1];
+    LzTok tok[LzShared<NT>::kWindow / 3 + 3];
+  } slot[2];
+  uint32_t warp_sum[NT / 32];
+};
+
+__device__ __forceinline__ void pair_barrier()
+{
+  asm volatile("barrier.cluster.arrive.release;\n\t"
+               "barrier.cluster.wait.acquire;" ::
+                 : "memory");
+}
+
+template<int NT>
+struct LzOther
+{
+  LzShared<NT>& S;
+  LzPairShared<NT>& P; // (in the second CTA's shared memory)
+  uint32_t turn;       // the slot being filled
+  __device__ LzTok* tok() { return P.slot[turn].tok; }
+  __device__ void post(const LzWork& q)
+  {
+    if (threadIdx.x == 0)
+      P.slot[turn].work = q;
+    pair_barrier();
+    turn ^= 1;
+  }
+  __device__ void tile(const uint8_t* lits, const uint8_t*, uint8_t* to, uint32_t nout)
+  {
+    for (uint32_t i = threadIdx.x; i < NT / 2 + 1; i += NT)
+      P.slot[turn].start[i] = S.t.tile.start[i];
+    post(LzWork{ LzWork::kTile, lits, to, nout, 0, 0 });
+  }
+  __device__ void run_long(const LzWork& q) { post(q); }
+};
+
+template<int NT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT)
+lz4_decode_pair_k(const uint8_t* in,
+                  const uint64_t* in_off,
+                  const uint64_t* in_size,
+                  uint64_t n_chunks,
+                  uint8_t* out,
+                  uint64_t out_stride,
+                  uint64_t chunk_bytes,
+                  uint32_t* status)
+{
+  CHUCKY_DYN_SHARED(uint4, sm);
+  const bool first = (blockIdx.x & 1) == 0;
+  pair_barrier(); // the second CTA's shared memory exists
+  uint32_t turn = 0;
+  for (uint64_t c = blockIdx.x >> 1; c < n_chunks; c += gridDim.x >> 1) {
+    if (first) {
+      LzShared<NT>& S = *reinterpret_cast<LzShared<NT>*>(sm);
+      uint64_t p = 0;
+      asm("mapa.u64 %0, %1, 1;" : "=l"(p) : "l"(reinterpret_cast<uint64_t>(sm)));
+      LzOther<NT> other{ S, *reinterpret_cast<LzPairShared<NT>*>(p), turn };
+      const uint8_t* src = in + in_off[c];
+      const uint64_t n = in_size[c];
+      uint8_t* dst = out + c * out_stride;
+      const bool ok = lz4_decode_tiles<NT>(S, other, src, n, dst, chunk_bytes);
+      __syncthreads(); // (a malformed block leaves from anywhere)
+      other.post(LzWork{ LzWork::kDone, nullptr, nullptr, 0, 0, 0 });
+      turn = other.turn;
+      // every tile is executed
+      if (threadIdx.x < 32) {
+        const uint32_t st =
+          ok ? uint32_t(kDecodeOk) : lz4_decode_serial(src, n, dst, chunk_bytes, int(threadIdx.x));
+        if (threadIdx.x == 0)
+          status[c] = st;
+      }
+      __syncthreads();
+    } else {
+      LzPairShared<NT>& P = *reinterpret_cast<LzPairShared<NT>*>(sm);
+      for (;;) {
+        pair_barrier();
+        const auto& slot = P.slot[turn];
+        turn ^= 1;
+        const LzWork q = slot.work;
+        if (q.kind == LzWork::kDone)
+          break;
+        if (q.kind == LzWork::kLong) {
+          lz4_copy_long<NT>(q);
+          continue;
+        }
+        for (uint32_t i = threadIdx.x; i < NT / 2 + 1; i += NT)
+          P.tile.start[i] = slot.start[i]; // (tile_run reads them behind a barrier)
+        tile_run<NT, 6>(P.tile, P.warp_sum, slot.tok, q.lits, q.to, uint32_t(q.lit));
+      }
+    }
+  }
+}
+
+template<int NT>
+cudaError_t launch_lz4_decode_pair(const uint8_t* in,
+                                   const uint64_t* in_off,
+                                   const uint64_t* in_size,
+                                   uint64_t n_chunks,
+                                   uint8_t* out,
+                                   uint64_t out_stride,
+                                   uint64_t chunk_bytes,
+                                   uint32_t* status,
+                                   cudaStream_t st)
+{
+  constexpr size_t smem = sizeof(LzShared<NT>) > sizeof(LzPairShared<NT>)
+                            ? sizeof(LzShared<NT>)
+                            : sizeof(LzPairShared<NT>);
+  const cudaError_t e = cudaFuncSetAttribute(
+    lz4_decode_pair_k<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (e != cudaSuccess)
+    return e;
+  lz4_decode_pair_k<NT><<<unsigned(2 * n_chunks), NT, smem, st>>>(
+    in, in_off, in_size, n_chunks, out, out_stride, chunk_bytes, status);
+  note_launches(1);
+  return cudaGetLastError();
+}
+#endif
 
 template<int NT>
 cudaError_t launch_lz4_decode_nt(const uint8_t* in,
@@ -559,7 +738,14 @@ cudaError_t launch_lz4_decode(const uint8_t* in,
 {
   // Chunks of up to 16 KiB: more CTAs of fewer threads, whose smaller tiles
   // suit them; larger ones: as many threads per tile as a CTA holds, since a
-  // chunk's tiles follow one another.
+  // chunk's tiles follow one another.  Where two CTAs per chunk still fit
+  // the chip side by side, the parse of a tile runs beside the execution of
+  // the one before: 1 to 76 sensor chunks of 1 MiB take 1.00 ms, 77 1.39.
+#ifndef CHUCKY_LZ4_UNPAIRED
+  if (chunk_bytes > kSmallChunk && n_chunks <= uint64_t(device_sm_count()) / 2)
+    return launch_lz4_decode_pair<CHUCKY_LZ4_THREADS>(in, in_off, in_size, n_chunks, out,
+                                                      out_stride, chunk_bytes, status, st);
+#endif
   return chunk_bytes <= kSmallChunk
            ? launch_lz4_decode_nt<CHUCKY_DECODE_THREADS>(in, in_off, in_size, n_chunks, out, out_stride,
                                        chunk_bytes, status, st)

@@ -272,6 +272,7 @@ inline cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t = null
 // decoders' CTAs of one or two warps: quicker here, and more tiles per chunk
 #define CHUCKY_DECODE_THREADS 64
 #define CHUCKY_LZ4_THREADS 64
+#define CHUCKY_LZ4_UNPAIRED
 #define CHUCKY_ZSTD_EXEC_THREADS 64
 #define CHUCKY_DECODE_WARPS 1
 

@@ -150,3 +150,35 @@ def test_malformed_blocks_keep_their_status(cap):
         assert s == want
         if want == 0:
             assert g.tobytes() == bytes(data)
+
+
+def check(blocks, cap):
+    st, got = run(blocks, cap)
+    for b, s, g in zip(blocks, st, got):
+        want, data = decode(b, cap)
+        assert s == want
+        if want == 0:
+            assert g.tobytes() == bytes(data)
+
+
+@pytest.mark.parametrize("cap", [16385, 60000])
+@pytest.mark.parametrize("n", [1, 2, 75, 76, 77, 160])
+def test_block_counts(n, cap):
+    """Two CTAs to a block, or one where there are more blocks than pairs."""
+    kinds = [make_block(cap, s, s % 2 == 1) for s in range(5)]
+    check([kinds[i % 5] for i in range(n)], cap)
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_few_malformed_blocks(seed):
+    """... of which some break off, and others are whole."""
+    cap, rng = 40000, np.random.default_rng(1000 + seed)
+    blocks = []
+    for s in range(8):
+        b = bytearray(make_block(cap, 10 * seed + s, s % 2 == 1))
+        if s % 4 == 1:
+            del b[int(rng.integers(0, len(b))):]
+        elif s % 4:
+            b[int(rng.integers(0, len(b)))] = int(rng.integers(0, 256))
+        blocks.append(bytes(b))
+    check(blocks, cap)
