@@ -265,7 +265,9 @@ __device__ __forceinline__ WideLane wide_lane(const WideWindow& W,
   L.cap = probe ? min(kLaneExtend - 1, end - q) : 0;
   L.need = ok ? len + 1 : 4;
   L.on = probe && L.need <= L.cap;
-  L.x2 = L.on ? word_at(words, q + L.need - 4) : 0;
+  L.x2 = x;
+  if (L.on && L.need > 4) // (most lanes of noisy data have no match to beat)
+    L.x2 = word_at(words, q + L.need - 4);
   return L;
 }
 
