@@ -366,9 +366,34 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint64_t ip = 0, op = 0;
   uint32_t want = Sh::kWindow; // window bytes worth parsing
+  bool peek = true;            // a long literal run may follow
+  auto run_long = [&](bool& last) {
+    LzWork q;
+    if (!lz4_long_sequence(S, src, n, dst, chunk_bytes, ip, op, last, q))
+      return false;
+    exec.run_long(q);
+    want = Sh::kWindow;
+    peek = true;
+    return true;
+  };
   for (;;) {
     if (ip >= n)
       return false;
+    if (peek) {
+      // a literal run that no window holds (an incompressible block is one)
+      // is known by its length bytes: no window is parsed for it
+      peek = false;
+      static_assert(kMaxExt == 32, "a lane per length byte");
+      const uint64_t at = ip + 1 + lane;
+      if (__all_sync(kAll, src[ip] >> 4 == 15 && at < n && src[at] == 255)) {
+        bool last = false;
+        if (!run_long(last))
+          return false;
+        if (last)
+          return op == chunk_bytes;
+        continue;
+      }
+    }
     const uint32_t wlen = uint32_t(n - ip < want ? n - ip : want);
     const bool at_end = ip + wlen == n;
     // ---- the window, in the 16-byte phase of the block
@@ -512,14 +537,11 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
         return false;
       if (used == 0) { // a sequence that fits neither window nor tile
         bool last = false;
-        LzWork q;
         __syncthreads(); // (S.bad and S.cut have been read)
-        if (!lz4_long_sequence(S, src, n, dst, chunk_bytes, ip, op, last, q))
+        if (!run_long(last))
           return false;
-        exec.run_long(q);
         if (last)
           return op == chunk_bytes;
-        want = Sh::kWindow;
         continue;
       }
       exec.tile(src + ip, b, dst + op, nout);
@@ -721,9 +743,6 @@ cudaError_t launch_lz4_decode_nt(const uint8_t* in,
   return cudaGetLastError();
 }
 
-// largest chunk of the small form
-constexpr uint64_t kSmallChunk = 16 << 10;
-
 } // namespace
 
 cudaError_t launch_lz4_decode(const uint8_t* in,
@@ -736,21 +755,34 @@ cudaError_t launch_lz4_decode(const uint8_t* in,
                               uint32_t* status,
                               cudaStream_t st)
 {
-  // Chunks of up to 16 KiB: more CTAs of fewer threads, whose smaller tiles
-  // suit them; larger ones: as many threads per tile as a CTA holds, since a
-  // chunk's tiles follow one another.  Where two CTAs per chunk still fit
-  // the chip side by side, the parse of a tile runs beside the execution of
-  // the one before: 1 to 76 sensor chunks of 1 MiB take 1.00 ms, 77 1.39.
+  // CTAs of 1,024 threads (one per SM) take the least time per chunk, CTAs of
+  // 256 (tiles of 4 KiB) keep more chunks on the chip.  Sensor chunks, us:
+  //   chunks x bytes      256  1,024  two CTAs
+  //      76 x 4,096        17     17     18
+  //      76 x 16,384       61     25     29
+  //      76 x 20,000       69     38     34
+  //      76 x 65,536      216     97     78
+  //     300 x 16,384       66     46    102
+  //     300 x 65,536      239    189    298
+  //     600 x 65,536      321    367    585
+  // (chunks that are part constant, part random: 300 x 16,384 60 and 62, 600 x
+  // 65,536 354 and 522.)  So: the small ones for chunks of one of their tiles,
+  // for chunks of one large tile when there are more than SMs, and for more
+  // than three waves of large ones; two CTAs per chunk where they fit the chip
+  // side by side and there is a second tile to parse ahead.
+  const uint64_t sms = uint64_t(device_sm_count());
+  constexpr uint64_t kSmallTile = CHUCKY_DECODE_THREADS * 16, kTile = CHUCKY_LZ4_THREADS * 16;
 #ifndef CHUCKY_LZ4_UNPAIRED
-  if (chunk_bytes > kSmallChunk && n_chunks <= uint64_t(device_sm_count()) / 2)
+  if (chunk_bytes > kTile && n_chunks <= sms / 2)
     return launch_lz4_decode_pair<CHUCKY_LZ4_THREADS>(in, in_off, in_size, n_chunks, out,
                                                       out_stride, chunk_bytes, status, st);
 #endif
-  return chunk_bytes <= kSmallChunk
-           ? launch_lz4_decode_nt<CHUCKY_DECODE_THREADS>(in, in_off, in_size, n_chunks, out, out_stride,
-                                       chunk_bytes, status, st)
-           : launch_lz4_decode_nt<CHUCKY_LZ4_THREADS>(in, in_off, in_size, n_chunks, out, out_stride,
-                                        chunk_bytes, status, st);
+  const bool small =
+    chunk_bytes <= kSmallTile || n_chunks > (chunk_bytes <= kTile ? sms : 3 * sms);
+  return small ? launch_lz4_decode_nt<CHUCKY_DECODE_THREADS>(in, in_off, in_size, n_chunks, out,
+                                                             out_stride, chunk_bytes, status, st)
+               : launch_lz4_decode_nt<CHUCKY_LZ4_THREADS>(in, in_off, in_size, n_chunks, out,
+                                                          out_stride, chunk_bytes, status, st);
 }
 
 } // namespace chucky

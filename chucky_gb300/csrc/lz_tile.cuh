@@ -13,7 +13,7 @@
 #include <stdint.h>
 
 // Threads of the decoders' CTAs (the CPU emulation of the kernels, where every
-// thread costs, has fewer): for chunks of up to 16 KiB, for larger ones, and
+// thread costs, has fewer): the small form, the large one, the zstd execution, and
 // warps where a warp works alone.
 #ifndef CHUCKY_DECODE_THREADS
 #define CHUCKY_DECODE_THREADS 256
