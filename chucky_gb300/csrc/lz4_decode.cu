@@ -594,7 +594,9 @@ lz4_decode_k(const uint8_t* in,
 // second executes a tile while the first parses the next.  A cluster barrier
 // per tile; both CTAs pass the same ones: the first ends its block with a
 // kDone of its own, the second leaves its loop only there.  Bound by the parse
-// and placement (12 of 20 us per tile), the longer half.
+// and placement (12 of 20 us per tile), the longer half; over both CTAs 43 % of
+// the issue slots are taken, and a third of the stalls are at the CTA's own
+// barriers.
 template<int NT>
 struct LzPairShared // the second CTA's
 {
