@@ -36,6 +36,17 @@ struct Pool
   cudaMemPool_t pool;
 };
 
+// While another stream is being captured (by this thread, or by any in the
+// global mode), making a pool, allocating from it and freeing count as unsafe
+// and would invalidate that capture.  Neither touches it: this thread says so
+// for the time of the call.
+struct CaptureRelaxed
+{
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 constexpr int kMaxPools = 64;
 std::mutex g_mutex;
 Pool g_pools[kMaxPools];
@@ -91,6 +102,7 @@ void* scratch_acquire(size_t bytes, cudaStream_t st)
   }
   if (cs != cudaStreamCaptureStatusNone)
     return nullptr;
+  const CaptureRelaxed relaxed;
   const cudaMemPool_t pool = pool_of_context(true);
   void* p = nullptr;
   if (!pool)
@@ -104,8 +116,10 @@ void* scratch_acquire(size_t bytes, cudaStream_t st)
 
 void scratch_release(void* p, cudaStream_t st)
 {
-  if (p)
-    cudaFreeAsync(p, st);
+  if (!p)
+    return;
+  const CaptureRelaxed relaxed;
+  cudaFreeAsync(p, st);
 }
 
 void scratch_trim()
