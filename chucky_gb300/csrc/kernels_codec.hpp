@@ -13,8 +13,8 @@ void note_launches(unsigned n);
 // Streaming multiprocessors of the current device.
 int device_sm_count();
 
-// Raw LZ4 blocks back to chunk bytes (a CTA per block, bounds-checked):
-// block i is in_size[i] bytes at in + in_off[i] and decodes to chunk_bytes
+// Raw LZ4 blocks back to chunk bytes (a warp, a CTA or two CTAs per block by
+// their number and size, bounds-checked): block i is in_size[i] bytes at in + in_off[i] and decodes to chunk_bytes
 // bytes at out + i * out_stride; status[i] 0 when it did exactly that.
 cudaError_t launch_lz4_decode(const uint8_t* in,
                               const uint64_t* in_off,

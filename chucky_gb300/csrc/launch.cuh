@@ -11,3 +11,10 @@
 #ifndef CHUCKY_DYN_SHARED
 #define CHUCKY_DYN_SHARED(T, name) extern __shared__ __align__(16) T name[]
 #endif
+
+// A device function that is called, for the sake of its caller's registers.
+#ifdef __CUDACC__
+#define CHUCKY_NOINLINE __noinline__
+#else
+#define CHUCKY_NOINLINE
+#endif

@@ -19,17 +19,18 @@
 //            an output tile;
 //   execute: every byte of the tile finds its value by following references
 //            to earlier bytes (lz_tile.cuh).
-// A sequence that does not fit a tile or whose length bytes run on (long
-// literal runs, long matches) is copied by the whole CTA.
+// A long sequence (literal run or match) is copied by the whole CTA.
 //
 // With few blocks two CTAs work on each, one parsing and placing ahead of the
-// other's execution (lz4_decode_pair_k).
+// other's execution (lz4_decode_pair_k).  With more blocks than the chip holds
+// CTAs, those of few sequences are decoded by a warp each, token by token:
+// there are enough of them to hide each other's latency (launch_lz4_decode).
 //
 // Bound by the integer instructions of the parse and of the tiles (about 20
-// us for a 16 KiB tile: 5 chain steps, 2 chain, 5 sequences, 8 tile), not by
-// memory: 64 sensor chunks of 1 MiB take 1.00 ms with two CTAs each, 1.39
-// with one (a warp per block, sequence by sequence: 62.3 ms), 1,024 of 16 KiB
-// 0.15 ms.
+// us for a 16 KiB tile: 12 of parse and placement, of them 5 chain steps, 2
+// chain, 5 sequences, and 8 tile), not by memory: 64 sensor chunks of 1 MiB take
+// 1.00 ms with two CTAs each, 1.39 with one (a warp per block, sequence by
+// sequence: 62.3 ms), 912 of 16 KiB 0.15 ms.
 //
 // Every read is checked against the block's size and every write against
 // the chunk size.  A block the fast path cannot finish is decoded once more
@@ -46,6 +47,13 @@ namespace chucky {
 
 namespace {
 
+// CTAs of the small form that an SM holds (64 registers a thread), and that
+// the chip does
+constexpr int kSmallCtas = 4;
+#ifndef CHUCKY_LZ4_SLOTS
+#define CHUCKY_LZ4_SLOTS(sms) (kSmallCtas * (sms))
+#endif
+
 enum : uint32_t
 {
   kDecodeOk = 0,
@@ -53,92 +61,133 @@ enum : uint32_t
   kDecodeBadOffset = 2, // a match offset of 0 or before the chunk start
   kDecodeOverrun = 3,   // the output would exceed the chunk size
   kDecodeShort = 4,     // the block ends before the chunk is complete
+  kDecodeLeft = 99,     // (not a status: left to the whole CTA)
 };
 
-// One block by one warp.  Every lane parses the same tokens (the byte loads
-// broadcast within the warp); literals are copied side by side, and a match
-// of offset d writes out[op + j] = out[op - d + j mod d] for j in
-// [0, length), which reads only bytes already final before op.
-__device__ uint32_t lz4_decode_serial(const uint8_t* src,
-                                      uint64_t n,
-                                      uint8_t* dst,
-                                      uint64_t chunk_bytes,
-                                      int lane)
+// Copies by one warp.
+__device__ __forceinline__ void warp_copy(uint8_t* dst, const uint8_t* src, uint64_t n)
 {
-  uint64_t ip = 0, op = 0;
-  uint32_t st = kDecodeOk;
-  while (true) {
-    if (ip >= n) {
-      st = kDecodeTruncated;
-      break;
-    }
-    const uint32_t token = src[ip++];
+  copy_exact(dst, src, n, threadIdx.x & 31, 32);
+}
+
+// A match by one warp (the bytes before `to` final and seen by all lanes): whole
+// periods of the offset first, then copies of doubling length.
+__device__ __forceinline__ void warp_match(uint8_t* to, uint32_t off, uint64_t ml)
+{
+  const uint8_t* const from = to - off;
+  const uint64_t first = off < 128 ? 128 / off * off : off;
+  uint64_t done = first < ml ? first : ml;
+  for (uint32_t j = threadIdx.x & 31; j < uint32_t(done); j += 32)
+    to[j] = from[j < off ? j : j % off];
+  while (done < ml) {
+    __syncwarp();
+    const uint64_t k = done < ml - done ? done : ml - done;
+    warp_copy(to + done, to, k);
+    done += k;
+  }
+}
+
+// A warp that may leave its block counts sequences by their bytes above
+// `worth`: once they fall kWorthLag sequences' worth behind (they get kWorthLead
+// ahead at most), or one has kLongSequence literals or match bytes, the rest is
+// left to the whole CTA.
+constexpr int kWorthLag = 3, kWorthLead = 32;
+constexpr uint32_t kLongSequence = 16 << 10;
+
+// One block by one warp, from ip and op on; `worth` 0: to its end, otherwise it
+// may be left at the sequence that ip and op then name.  Every lane parses the
+// same tokens (the byte loads broadcast within the warp); a match reads only
+// bytes already final before op.  kVec: copies by vectors where they are long
+// (the code for it costs a short kernel more than it gives).
+template<bool kVec>
+__device__ __forceinline__ uint32_t lz4_decode_warp(const uint8_t* src,
+                                                    uint64_t n,
+                                                    uint8_t* dst,
+                                                    uint64_t chunk_bytes,
+                                                    int worth,
+                                                    uint64_t& ip,
+                                                    uint64_t& op)
+{
+  const uint32_t lane = threadIdx.x & 31;
+  int lead = 0;
+  for (;;) {
+    uint64_t at = ip, to = op; // (the sequence is taken once it is done)
+    if (at >= n)
+      return kDecodeTruncated;
+    const uint32_t token = src[at++];
     uint64_t lit = token >> 4;
-    if (lit == 15) {
-      uint32_t b = 255;
-      while (b == 255) {
-        if (ip >= n) {
-          st = kDecodeTruncated;
-          break;
-        }
-        b = src[ip++];
-        lit += b;
+    if (lit == 15)
+      for (uint32_t b = 255; b == 255; lit += b) {
+        if (at >= n)
+          return kDecodeTruncated;
+        b = src[at++];
       }
-      if (st)
-        break;
-    }
-    if (lit > n - ip) {
-      st = kDecodeTruncated;
-      break;
-    }
-    if (lit > chunk_bytes - op) {
-      st = kDecodeOverrun;
-      break;
-    }
-    for (uint64_t j = lane; j < lit; j += 32)
-      dst[op + j] = src[ip + j];
-    ip += lit;
-    op += lit;
-    if (ip == n) // the last sequence has literals only
-      break;
-    if (n - ip < 2) {
-      st = kDecodeTruncated;
-      break;
-    }
-    const uint64_t off = uint64_t(src[ip]) | uint64_t(src[ip + 1]) << 8;
-    ip += 2;
-    if (off == 0 || off > op) {
-      st = kDecodeBadOffset;
-      break;
-    }
+    if (worth && lit >= kLongSequence)
+      return kDecodeLeft;
+    if (lit > n - at)
+      return kDecodeTruncated;
+    if (lit > chunk_bytes - to)
+      return kDecodeOverrun;
+    if (kVec && lit >= 256)
+      warp_copy(dst + to, src + at, lit);
+    else
+      for (uint64_t j = lane; j < lit; j += 32)
+        dst[to + j] = src[at + j];
+    at += lit;
+    to += lit;
+    if (at == n) // the last sequence has literals only
+      return to == chunk_bytes ? kDecodeOk : kDecodeShort;
+    if (n - at < 2)
+      return kDecodeTruncated;
+    const uint32_t off = src[at] | uint32_t(src[at + 1]) << 8;
+    at += 2;
+    if (off == 0 || off > to)
+      return kDecodeBadOffset;
     uint64_t ml = (token & 15) + 4;
-    if ((token & 15) == 15) {
-      uint32_t b = 255;
-      while (b == 255) {
-        if (ip >= n) {
-          st = kDecodeTruncated;
-          break;
-        }
-        b = src[ip++];
-        ml += b;
+    if ((token & 15) == 15)
+      for (uint32_t b = 255; b == 255; ml += b) {
+        if (at >= n)
+          return kDecodeTruncated;
+        b = src[at++];
       }
-      if (st)
-        break;
-    }
-    if (ml > chunk_bytes - op) {
-      st = kDecodeOverrun;
-      break;
-    }
+    if (worth && ml >= kLongSequence)
+      return kDecodeLeft; // (its literals are written once more)
+    if (ml > chunk_bytes - to)
+      return kDecodeOverrun;
     // the literals just written by other lanes are read below
     __syncwarp();
-    const uint8_t* m = dst + op - off;
-    for (uint64_t j = lane; j < ml; j += 32)
-      dst[op + j] = m[j < off ? j : j % off];
+    if (kVec && ml >= 256) {
+      warp_match(dst + to, off, ml);
+    } else {
+      const uint8_t* m = dst + to - off;
+      for (uint64_t j = lane; j < ml; j += 32)
+        dst[to + j] = m[j < off ? j : j % off];
+    }
     __syncwarp();
-    op += ml;
+    const uint64_t made = to + ml - op;
+    ip = at;
+    op = to + ml;
+    if (worth) {
+      lead = min(lead + int(min(made, uint64_t(65536))) - worth, kWorthLead * worth);
+      if (lead < -kWorthLag * worth)
+        return kDecodeLeft;
+    }
   }
-  if (st == kDecodeOk && op != chunk_bytes)
-    st = kDecodeShort;
+}
+
+// ... called, for the registers of the kernels of whole CTAs
+__device__ CHUCKY_NOINLINE uint32_t lz4_decode_serial(const uint8_t* src,
+                                                      uint64_t n,
+                                                      uint8_t* dst,
+                                                      uint64_t chunk_bytes,
+                                                      int worth,
+                                                      uint64_t& ip_out,
+                                                      uint64_t& op_out)
+{
+  uint64_t ip = 0, op = 0;
+  const uint32_t st = lz4_decode_warp<true>(src, n, dst, chunk_bytes, worth, ip, op);
+  ip_out = ip;
+  op_out = op;
   return st;
 }
 
@@ -149,6 +198,18 @@ constexpr uint32_t kWarpSpan = 512; // window positions per warp
 static_assert(kWarpSpan == 32 * kPer, "a warp's threads share its span");
 // length bytes of one field followed inside a window (each adds 255)
 constexpr uint32_t kMaxExt = 32;
+// ... and those of one that is copied without a window being parsed: a length
+// of 525 in a small tile, 2,055 in a large one, which holds several such; in a
+// block of half a small tile, whose window is parsed anyway, most of the block.
+// 300 blocks of 16 KiB that are constant or random take 23 us in small tiles
+// (62 with random ones of 8 KiB and up taken so).
+template<int NT>
+__device__ __forceinline__ uint32_t lz4_peek_bytes(uint64_t chunk_bytes)
+{
+  if (NT <= 256 && chunk_bytes <= 2048)
+    return (uint32_t(chunk_bytes) * 3 / 4 + 239) / 255;
+  return NT <= 256 ? 2 : 8;
+}
 // where the chain goes from a position: the next token's position, or
 constexpr uint32_t kStop = 0x8000;  // | position: that token is not complete here
 constexpr uint32_t kEnd = 0xFFFE;   // the block's last sequence
@@ -351,22 +412,23 @@ struct LzOwn
   __device__ void run_long(const LzWork& q) { lz4_copy_long<NT>(q); }
 };
 
-// `n` bytes of a block at src by all NT threads; false when it is malformed.
-// X: who executes the tiles.
+// `n` bytes of a block at src by all NT threads, from ip and op on; false when
+// it is malformed.  X: who executes the tiles.
 template<int NT, typename X>
 __device__ bool lz4_decode_tiles(LzShared<NT>& S,
                                  X& exec,
                                  const uint8_t* src,
                                  const uint64_t n,
                                  uint8_t* dst,
-                                 const uint64_t chunk_bytes)
+                                 const uint64_t chunk_bytes,
+                                 uint64_t ip = 0,
+                                 uint64_t op = 0)
 {
   using Sh = LzShared<NT>;
   constexpr unsigned kAll = 0xffffffffu;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint64_t ip = 0, op = 0;
   uint32_t want = Sh::kWindow; // window bytes worth parsing
-  bool peek = true;            // a long literal run may follow
+  bool peek = true;            // a long sequence may follow
   auto run_long = [&](bool& last) {
     LzWork q;
     if (!lz4_long_sequence(S, src, n, dst, chunk_bytes, ip, op, last, q))
@@ -380,12 +442,15 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
     if (ip >= n)
       return false;
     if (peek) {
-      // a literal run that no window holds (an incompressible block is one)
-      // is known by its length bytes: no window is parsed for it
+      // a long literal run (an incompressible block is one) and a long match
+      // behind a few literals (constant data is one after another) are known
+      // by their length bytes: no window is parsed for them
       peek = false;
-      static_assert(kMaxExt == 32, "a lane per length byte");
-      const uint64_t at = ip + 1 + lane;
-      if (__all_sync(kAll, src[ip] >> 4 == 15 && at < n && src[at] == 255)) {
+      const uint32_t t = src[ip], lit = t >> 4;
+      const bool run = lit == 15;
+      const uint64_t at = ip + 1 + (run ? 0 : lit + 2) + lane;
+      const bool full = lane >= lz4_peek_bytes<NT>(chunk_bytes) || (at < n && src[at] == 255);
+      if (__all_sync(kAll, full && (run || (t & 15) == 15))) {
         bool last = false;
         if (!run_long(last))
           return false;
@@ -558,8 +623,30 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
   }
 }
 
-template<int NT>
-__global__ void __launch_bounds__(NT)
+// Whether a block has few sequences, by its size: it saved less than a 64th of
+// its bytes (matches are rare), or takes less than an eighth (a sequence is
+// three bytes or more).  Not one that starts with kLongSequence literals, which
+// a CTA copies sooner.
+__device__ __forceinline__ bool lz4_few_sequences(const uint8_t* src, uint64_t n, uint64_t chunk_bytes)
+{
+  if (n < chunk_bytes - chunk_bytes / 64)
+    return n < chunk_bytes / 8;
+  constexpr uint32_t kBytes = kLongSequence / 255 + 1;
+  static_assert(kBytes > 32 && kBytes <= 96, "two or three length bytes per lane");
+  const uint32_t lane = threadIdx.x & 31;
+  bool full = n > kBytes && src[0] >> 4 == 15;
+  for (uint32_t k = lane; k < kBytes && full; k += 32)
+    full = src[1 + k] == 255;
+  return !__all_sync(0xffffffffu, full);
+}
+
+// kMany: CTAs below `groups` take `per` blocks each (a warp a block at most): the
+// warps decode those of few sequences alone, as far as that is worth it, and the
+// CTA then goes over what they left.  The others take one of the remaining
+// blocks each.  A warp needs no barriers, and the chip holds 32 of them per SM,
+// but it waits 0.3 to 0.65 us for every sequence.
+template<int NT, bool kMany>
+__global__ void __launch_bounds__(NT, NT <= 256 ? kSmallCtas : 1)
 lz4_decode_k(const uint8_t* in,
              const uint64_t* in_off,
              const uint64_t* in_size,
@@ -567,24 +654,84 @@ lz4_decode_k(const uint8_t* in,
              uint8_t* out,
              uint64_t out_stride,
              uint64_t chunk_bytes,
-             uint32_t* status)
+             uint32_t* status,
+             uint32_t groups,
+             uint32_t per,
+             int worth)
 {
   CHUCKY_DYN_SHARED(uint4, sm);
   LzShared<NT>& S = *reinterpret_cast<LzShared<NT>*>(sm);
-  for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
+  __shared__ uint64_t left_ip[NT / 32], left_op[NT / 32];
+  __shared__ uint32_t left[NT / 32];
+  auto block = [&](uint64_t c, uint64_t ip, uint64_t op) {
     const uint8_t* src = in + in_off[c];
     const uint64_t n = in_size[c];
     uint8_t* dst = out + c * out_stride;
     LzOwn<NT> own{ S };
-    const bool ok = lz4_decode_tiles<NT>(S, own, src, n, dst, chunk_bytes);
+    const bool ok = lz4_decode_tiles<NT>(S, own, src, n, dst, chunk_bytes, ip, op);
     __syncthreads();
     if (threadIdx.x < 32) {
+      uint64_t ip0 = 0, op0 = 0;
       const uint32_t st =
-        ok ? uint32_t(kDecodeOk) : lz4_decode_serial(src, n, dst, chunk_bytes, int(threadIdx.x));
+        ok ? uint32_t(kDecodeOk) : lz4_decode_serial(src, n, dst, chunk_bytes, 0, ip0, op0);
       if (threadIdx.x == 0)
         status[c] = st;
     }
     __syncthreads();
+  };
+  if constexpr (kMany) {
+    __shared__ uint64_t left_ip[NT / 32], left_op[NT / 32];
+    __shared__ uint32_t left[NT / 32];
+    const uint32_t warp = threadIdx.x >> 5;
+    const bool group = blockIdx.x < groups;
+    const uint64_t c0 = group ? uint64_t(blockIdx.x) * per : uint64_t(blockIdx.x - groups);
+    const uint32_t m = !group ? 1 : uint32_t(n_chunks - c0 < per ? n_chunks - c0 : per);
+    if (warp < m) {
+      const uint64_t c = c0 + warp, n = in_size[c];
+      const uint8_t* src = in + in_off[c];
+      const bool few = lz4_few_sequences(src, n, chunk_bytes);
+      uint64_t ip = 0, op = 0;
+      uint32_t st = group == few ? kDecodeLeft : kDecodeOk; // (Ok: another CTA's block)
+      if (group && few) {
+        st = lz4_decode_serial(src, n, out + c * out_stride, chunk_bytes, worth, ip, op);
+        if (st != kDecodeLeft && (threadIdx.x & 31) == 0)
+          status[c] = st;
+      }
+      if ((threadIdx.x & 31) == 0) {
+        left_ip[warp] = ip;
+        left_op[warp] = op;
+        left[warp] = st;
+      }
+    }
+    __syncthreads();
+    for (uint32_t k = 0; k < m; ++k)
+      if (left[k] == kDecodeLeft) // (the whole CTA)
+        block(c0 + k, left_ip[k], left_op[k]);
+  } else {
+    for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x)
+      block(c, 0, 0);
+  }
+}
+
+// A warp per block, for chunks too small for more.
+constexpr int kAloneThreads = 128;
+__global__ void __launch_bounds__(kAloneThreads) lz4_decode_alone_k(const uint8_t* in,
+                                                                    const uint64_t* in_off,
+                                                                    const uint64_t* in_size,
+                                                                    uint64_t n_chunks,
+                                                                    uint8_t* out,
+                                                                    uint64_t out_stride,
+                                                                    uint64_t chunk_bytes,
+                                                                    uint32_t* status)
+{
+  constexpr uint32_t kWarps = kAloneThreads / 32;
+  for (uint64_t c = uint64_t(blockIdx.x) * kWarps + (threadIdx.x >> 5); c < n_chunks;
+       c += uint64_t(gridDim.x) * kWarps) {
+    uint64_t ip = 0, op = 0;
+    const uint32_t st = lz4_decode_warp<false>(in + in_off[c], in_size[c], out + c * out_stride,
+                                               chunk_bytes, 0, ip, op);
+    if ((threadIdx.x & 31) == 0)
+      status[c] = st;
   }
 }
 
@@ -670,8 +817,10 @@ lz4_decode_pair_k(const uint8_t* in,
       turn = other.turn;
       // every tile is executed
       if (threadIdx.x < 32) {
+        uint64_t ip = 0, op = 0;
         const uint32_t st =
-          ok ? uint32_t(kDecodeOk) : lz4_decode_serial(src, n, dst, chunk_bytes, int(threadIdx.x));
+          ok ? uint32_t(kDecodeOk)
+             : lz4_decode_serial(src, n, dst, chunk_bytes, 0, ip, op);
         if (threadIdx.x == 0)
           status[c] = st;
       }
@@ -722,7 +871,7 @@ cudaError_t launch_lz4_decode_pair(const uint8_t* in,
 }
 #endif
 
-template<int NT>
+template<int NT, bool kMany>
 cudaError_t launch_lz4_decode_nt(const uint8_t* in,
                                  const uint64_t* in_off,
                                  const uint64_t* in_size,
@@ -731,16 +880,19 @@ cudaError_t launch_lz4_decode_nt(const uint8_t* in,
                                  uint64_t out_stride,
                                  uint64_t chunk_bytes,
                                  uint32_t* status,
+                                 uint32_t per,
+                                 int worth,
                                  cudaStream_t st)
 {
   constexpr size_t smem = sizeof(LzShared<NT>);
   const cudaError_t e = cudaFuncSetAttribute(
-    lz4_decode_k<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    lz4_decode_k<NT, kMany>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess)
     return e;
-  const uint64_t grid = n_chunks < 0x7FFFFFFFull ? n_chunks : 0x7FFFFFFFull;
-  CHUCKY_LAUNCH(lz4_decode_k<NT>, unsigned(grid), NT, smem, st, in, in_off, in_size, n_chunks,
-                out, out_stride, chunk_bytes, status);
+  const uint64_t groups = kMany ? (n_chunks + per - 1) / per : 0, ctas = groups + n_chunks;
+  const uint64_t grid = ctas < 0x7FFFFFFFull ? ctas : 0x7FFFFFFFull;
+  CHUCKY_LAUNCH((lz4_decode_k<NT, kMany>), unsigned(grid), NT, smem, st, in, in_off, in_size,
+                n_chunks, out, out_stride, chunk_bytes, status, uint32_t(groups), per, worth);
   note_launches(1);
   return cudaGetLastError();
 }
@@ -758,33 +910,63 @@ cudaError_t launch_lz4_decode(const uint8_t* in,
                               cudaStream_t st)
 {
   // CTAs of 1,024 threads (one per SM) take the least time per chunk, CTAs of
-  // 256 (tiles of 4 KiB) keep more chunks on the chip.  Sensor chunks, us:
-  //   chunks x bytes      256  1,024  two CTAs
-  //      76 x 4,096        17     17     18
-  //      76 x 16,384       61     25     29
-  //      76 x 20,000       69     38     34
-  //      76 x 65,536      216     97     78
-  //     300 x 16,384       66     46    102
-  //     300 x 65,536      239    189    298
-  //     600 x 65,536      321    367    585
-  // (chunks that are part constant, part random: 300 x 16,384 60 and 62, 600 x
-  // 65,536 354 and 522.)  So: the small ones for chunks of one of their tiles,
-  // for chunks of one large tile when there are more than SMs, and for more
-  // than three waves of large ones; two CTAs per chunk where they fit the chip
-  // side by side and there is a second tile to parse ahead.
-  const uint64_t sms = uint64_t(device_sm_count());
-  constexpr uint64_t kSmallTile = CHUCKY_DECODE_THREADS * 16, kTile = CHUCKY_LZ4_THREADS * 16;
+  // 256 (tiles of 4 KiB) keep more chunks on the chip.  us, for sensor counts, a
+  // textured volume (rare matches), noise, and chunks that are constant or
+  // random:
+  //   chunks x bytes   256                1,024              two CTAs
+  //      64 x 4,096     19  24  10  14     18  18  10  15
+  //      64 x 16,384    64  65  10  21     27  33  10  24
+  //      64 x 65,536   222 205  11  55     97  90  11  52     79  70  11  44
+  //     300 x 16,384    69  69  10  24     48  59  35  40
+  //     300 x 65,536   243 222  13  60    190 174  16  97
+  //     456 x 65,536   276 249  16  68    281 257  23 141
+  // So: the small ones for chunks of one of their tiles, for chunks of one large
+  // tile when there are more than SMs (each form is the better one for half of
+  // the data there), and for more than two waves of larger ones; two CTAs per
+  // chunk where they fit the chip side by side and there is a second tile to
+  // parse ahead.
+  //
+  // From two waves of small CTAs on (four per SM; from one for chunks up to 1
+  // KiB) warps decode the blocks of few sequences first; with fewer blocks a
+  // wave of CTAs is as quick.  A sequence must be worth its 0.65 us, with 32
+  // warps on an SM, against the CTA's 4.7 us per KiB of each of its chunks.
+  // us, every chunk to a CTA / so / every chunk to a warp:
+  //   chunks x bytes     sensor counts   volume           constant or random
+  //   1,467 x 4,440       80  82  260     72  38  41      76  18  33
+  //   4,096 x 4,096      127 132  325    149  44  41     141  23  36
+  //   4,096 x 8,192      279 288  715    251  86  84     204  29  64
+  //   2,048 x 16,384     288 294 1114    247 144 146     199  37  95
+  // Chunks of up to 512 bytes are all left to single warps (608 of 256 bytes: 3.3
+  // us on the device, 9.2 with CTAs; 64 sensor ones of 500 bytes 13.5 and 10.6),
+  // and so are many of up to 1 KiB (4,096 of sensor counts: 54 and 82 us).
+  const uint64_t sms = uint64_t(device_sm_count()), slots = CHUCKY_LZ4_SLOTS(sms);
+  constexpr int kSmallNT = CHUCKY_DECODE_THREADS, kNT = CHUCKY_LZ4_THREADS;
+  constexpr uint64_t kSmallTile = kSmallNT * 16, kTile = kNT * 16;
+  if (chunk_bytes <= 512 || (chunk_bytes <= 1024 && n_chunks > 3 * slots)) {
+    constexpr uint32_t kWarps = kAloneThreads / 32;
+    const uint64_t ctas = (n_chunks + kWarps - 1) / kWarps;
+    CHUCKY_LAUNCH(lz4_decode_alone_k, unsigned(ctas < 0x7FFFFFFFull ? ctas : 0x7FFFFFFFull),
+                  kAloneThreads, 0, st, in, in_off, in_size, n_chunks, out, out_stride,
+                  chunk_bytes, status);
+    note_launches(1);
+    return cudaGetLastError();
+  }
 #ifndef CHUCKY_LZ4_UNPAIRED
   if (chunk_bytes > kTile && n_chunks <= sms / 2)
-    return launch_lz4_decode_pair<CHUCKY_LZ4_THREADS>(in, in_off, in_size, n_chunks, out,
-                                                      out_stride, chunk_bytes, status, st);
+    return launch_lz4_decode_pair<kNT>(in, in_off, in_size, n_chunks, out, out_stride,
+                                       chunk_bytes, status, st);
 #endif
-  const bool small =
-    chunk_bytes <= kSmallTile || n_chunks > (chunk_bytes <= kTile ? sms : 3 * sms);
-  return small ? launch_lz4_decode_nt<CHUCKY_DECODE_THREADS>(in, in_off, in_size, n_chunks, out,
-                                                             out_stride, chunk_bytes, status, st)
-               : launch_lz4_decode_nt<CHUCKY_LZ4_THREADS>(in, in_off, in_size, n_chunks, out,
-                                                          out_stride, chunk_bytes, status, st);
+  if (chunk_bytes > kSmallTile && n_chunks <= (chunk_bytes <= kTile ? sms : 2 * sms))
+    return launch_lz4_decode_nt<kNT, false>(in, in_off, in_size, n_chunks, out, out_stride,
+                                            chunk_bytes, status, 1, 0, st);
+  if (n_chunks <= (chunk_bytes <= 1024 ? 1 : 2) * slots || n_chunks >= (1ull << 30))
+    return launch_lz4_decode_nt<kSmallNT, false>(in, in_off, in_size, n_chunks, out, out_stride,
+                                                 chunk_bytes, status, 1, 0, st);
+  const uint64_t share = (n_chunks + slots - 1) / slots;
+  const uint32_t per = uint32_t(share < kSmallNT / 32 ? share : kSmallNT / 32);
+  return launch_lz4_decode_nt<kSmallNT, true>(in, in_off, in_size, n_chunks, out, out_stride,
+                                              chunk_bytes, status, per,
+                                              160 / int(per > 2 ? per - 1 : 1), st);
 }
 
 } // namespace chucky

@@ -68,14 +68,17 @@ __device__ __forceinline__ T cta_scan(T v, T* warp_sum, T& total)
 
 // A match of any length by the whole CTA: `ml` bytes at `to` from `off`
 // bytes back (both final before it; a barrier before the call).  The first
-// 64 periods byte by byte, then copies of doubling length from the bytes
-// already written, which lie a multiple of the offset behind.
+// 64 periods, or 16 bytes per thread, byte by byte, then copies of doubling
+// length from the bytes already written, which lie a multiple of the offset
+// behind.
 template<int NT>
 __device__ void cta_match(uint8_t* to, uint64_t off, uint64_t ml)
 {
-  uint64_t done = off * 64 < ml ? off * 64 : ml;
-  for (uint64_t j = threadIdx.x; j < done; j += NT)
-    to[j] = (to - off)[j < off ? j : j % off];
+  const uint64_t first = off * 64 < NT * 16 ? NT * 16 / off * off : off * 64;
+  uint64_t done = first < ml ? first : ml; // (below 2^32: ml or 64 offsets are)
+  const uint32_t period = uint32_t(off);
+  for (uint32_t j = threadIdx.x; j < uint32_t(done); j += NT)
+    to[j] = (to - off)[j < period ? j : j % period];
   while (done < ml) {
     __syncthreads();
     const uint64_t k = done < ml - done ? done : ml - done;
