@@ -14,8 +14,9 @@ void note_launches(unsigned n);
 int device_sm_count();
 
 // Raw LZ4 blocks back to chunk bytes (a warp, a CTA or two CTAs per block by
-// their number and size, bounds-checked): block i is in_size[i] bytes at in + in_off[i] and decodes to chunk_bytes
-// bytes at out + i * out_stride; status[i] 0 when it did exactly that.
+// their number and size, bounds-checked): block i is in_size[i] bytes at
+// in + in_off[i] and decodes to chunk_bytes bytes at out + i * out_stride;
+// status[i] 0 when it did exactly that.
 cudaError_t launch_lz4_decode(const uint8_t* in,
                               const uint64_t* in_off,
                               const uint64_t* in_size,

@@ -846,12 +846,13 @@ cudaError_t launch_zstd_decode(const uint8_t* in,
   if (!n_chunks)
     return cudaSuccess;
   // chunks per launch set: as many as the kept scratch has lists for
-  const uint64_t one = zd_bytes(1, chunk_bytes);
+  const uint64_t one = zd_list_bytes(chunk_bytes);
   uint64_t wave = kZdScratch / one;
   wave = wave < 1 ? 1 : wave > n_chunks ? n_chunks : wave;
+  const uint64_t group = n_chunks < kZdFrames ? n_chunks : kZdFrames;
   uint8_t* const scratch =
     chunk_bytes < (1ull << 32)
-      ? static_cast<uint8_t*>(scratch_acquire(zd_bytes(wave, chunk_bytes), st))
+      ? static_cast<uint8_t*>(scratch_acquire(wave * one + group * sizeof(ZFrame), st))
       : nullptr;
   cudaError_t e = cudaSuccess;
   if (!scratch) {
@@ -860,26 +861,34 @@ cudaError_t launch_zstd_decode(const uint8_t* in,
                   out_stride, chunk_bytes, status, static_cast<const ZFrame*>(nullptr));
     return cudaGetLastError();
   }
-  for (uint64_t f = 0; f < n_chunks && e == cudaSuccess; f += wave) {
+  // Launch sets one after the other; what they leave is decoded once all are
+  // through, a frame's time for all of it and not for every set.
+  for (uint64_t g = 0; g < n_chunks && e == cudaSuccess; g += group) {
+    const uint64_t end = n_chunks - g < group ? n_chunks : g + group;
     ZWave W{};
     W.in = in;
-    W.in_off = in_off + f;
-    W.in_size = in_size + f;
-    W.out = out + f * out_stride;
     W.out_stride = out_stride;
     W.chunk_bytes = chunk_bytes;
-    W.status = status + f;
-    W.n = n_chunks - f < wave ? n_chunks - f : wave;
     W.max_blk = zd_max_blk(chunk_bytes);
     W.max_seq = zd_max_seq(chunk_bytes);
     W.seqs = reinterpret_cast<uint64_t*>(scratch);
     W.blocks = reinterpret_cast<ZBlk*>(W.seqs + wave * W.max_seq);
-    W.frames = reinterpret_cast<ZFrame*>(W.blocks + wave * W.max_blk);
-    if ((e = zd_launch(W, st)) != cudaSuccess)
+    ZFrame* const frames = reinterpret_cast<ZFrame*>(W.blocks + wave * W.max_blk);
+    for (uint64_t f = g; f < end && e == cudaSuccess; f += wave) {
+      W.in_off = in_off + f;
+      W.in_size = in_size + f;
+      W.out = out + f * out_stride;
+      W.status = status + f;
+      W.n = end - f < wave ? end - f : wave;
+      W.frames = frames + (f - g);
+      e = zd_launch(W, st);
+    }
+    if (e != cudaSuccess)
       break;
     note_launches(1);
-    CHUCKY_LAUNCH(zstd_decode_k, unsigned(W.n), 32, 0, st, in, W.in_off, W.in_size, W.out,
-                  out_stride, chunk_bytes, W.status, static_cast<const ZFrame*>(W.frames));
+    CHUCKY_LAUNCH(zstd_decode_k, unsigned(end - g), 32, 0, st, in, in_off + g, in_size + g,
+                  out + g * out_stride, out_stride, chunk_bytes, status + g,
+                  static_cast<const ZFrame*>(frames));
     e = cudaGetLastError();
   }
   scratch_release(scratch, st);

@@ -84,17 +84,24 @@ struct ZWave // one launch set's chunks and lists
   uint32_t max_blk, max_seq;
 };
 
-// scratch of one launch set
-constexpr uint64_t kZdScratch = 256ull << 20;
+// lists of one launch set
+#ifndef CHUCKY_ZSTD_SCRATCH
+#define CHUCKY_ZSTD_SCRATCH (256ull << 20)
+#endif
+constexpr uint64_t kZdScratch = CHUCKY_ZSTD_SCRATCH;
+// chunks whose frames' records are kept for one pass of the sequential decoder
+#ifndef CHUCKY_ZSTD_FRAMES
+#define CHUCKY_ZSTD_FRAMES (1ull << 20)
+#endif
+constexpr uint64_t kZdFrames = CHUCKY_ZSTD_FRAMES;
 
 // Lists of a frame: blocks of 4 KiB on average or more (the format allows
 // less), sequences of 4 bytes on average or more.
 inline uint32_t zd_max_blk(uint64_t chunk_bytes) { return uint32_t(chunk_bytes >> 12) + 16; }
 inline uint32_t zd_max_seq(uint64_t chunk_bytes) { return uint32_t(chunk_bytes >> 2) + 64; }
-inline uint64_t zd_bytes(uint64_t n, uint64_t chunk_bytes)
+inline uint64_t zd_list_bytes(uint64_t chunk_bytes)
 {
-  return n * (sizeof(ZFrame) + zd_max_blk(chunk_bytes) * sizeof(ZBlk) +
-              zd_max_seq(chunk_bytes) * 8ull) + 256;
+  return zd_max_blk(chunk_bytes) * sizeof(ZBlk) + zd_max_seq(chunk_bytes) * 8ull;
 }
 
 // A sequence in the list: literals (17 bits), match length (18), offset
