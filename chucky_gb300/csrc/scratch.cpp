@@ -124,6 +124,7 @@ void scratch_release(void* p, cudaStream_t st)
 
 void scratch_trim()
 {
+  const CaptureRelaxed relaxed;
   const cudaMemPool_t pool = pool_of_context(false);
   if (pool && cudaMemPoolTrimTo(pool, 0) != cudaSuccess)
     cudaGetLastError();

@@ -8,7 +8,7 @@
 namespace chucky {
 
 // What the pool keeps between calls at most (more is handed back to the
-// device when its work is done).  Mapping device memory afresh costs a call
+// device at the next synchronization after its work is done).  Mapping device memory afresh costs a call
 // hundreds of microseconds.
 constexpr size_t kScratchKept = size_t(256) << 20;
 
@@ -24,5 +24,9 @@ void scratch_trim();
 // The ID of the calling thread's current context (never reused), 0: unknown.
 unsigned long long current_context_id();
 
+} // namespace chucky
+#else
+namespace chucky {
+inline void scratch_trim() {}
 } // namespace chucky
 #endif

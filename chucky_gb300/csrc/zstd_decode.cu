@@ -845,15 +845,20 @@ cudaError_t launch_zstd_decode(const uint8_t* in,
 {
   if (!n_chunks)
     return cudaSuccess;
-  // chunks per launch set: as many as the kept scratch has lists for
+  // chunks per launch set: as many as the kept scratch has lists for, fewer
+  // where the device has no room for that many (a chunk above about 120 MiB
+  // needs more than the kept scratch for itself)
   const uint64_t one = zd_list_bytes(chunk_bytes);
+  const uint64_t group = n_chunks < kZdFrames ? n_chunks : kZdFrames;
   uint64_t wave = kZdScratch / one;
   wave = wave < 1 ? 1 : wave > n_chunks ? n_chunks : wave;
-  const uint64_t group = n_chunks < kZdFrames ? n_chunks : kZdFrames;
-  uint8_t* const scratch =
-    chunk_bytes < (1ull << 32)
-      ? static_cast<uint8_t*>(scratch_acquire(wave * one + group * sizeof(ZFrame), st))
-      : nullptr;
+  uint8_t* scratch = nullptr;
+  if (chunk_bytes < (1ull << 32))
+    for (;; wave = (wave + 3) / 4) {
+      scratch = static_cast<uint8_t*>(scratch_acquire(wave * one + group * sizeof(ZFrame), st));
+      if (scratch || wave == 1)
+        break;
+    }
   cudaError_t e = cudaSuccess;
   if (!scratch) {
     note_launches(1);
@@ -908,8 +913,10 @@ chucky_zstd_decode_chunks(const void* d_in,
                           uint32_t* d_status,
                           void* cuda_stream)
 {
-  if (!n_chunks)
+  if (!n_chunks) {
+    chucky::scratch_trim();
     return 0;
+  }
   if (!d_in || !d_in_offsets || !d_in_sizes || !d_out || !d_status ||
       out_stride < chunk_bytes || n_chunks > 0x7FFFFFFFu)
     return 1;

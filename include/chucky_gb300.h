@@ -188,9 +188,12 @@ extern "C"
    * frame is never read or written out of bounds.  Runs asynchronously on
    * `cuda_stream` (a cudaStream_t; NULL for the default stream).  The
    * blocks of a chunk are decoded side by side with device scratch from a
-   * pool of the library's own (about twice the output, 256 MiB at most at a
-   * time; what the pool keeps is handed back when a stream is destroyed);
-   * where there is none to be had -- no memory left, the stream being
+   * pool of the library's own: per call in flight about twice the output, in
+   * sets of 256 MiB and 16 bytes a chunk at most (a chunk above 120 MiB takes
+   * about twice its size), and smaller sets where the device has no room for
+   * that.  Up to 256 MiB stay in the pool between calls; they are handed back
+   * when a stream is destroyed and by a call with n_chunks 0.  Where there is
+   * no scratch to be had -- no memory left, the stream being
    * captured -- each chunk is decoded sequentially by one thread, with the
    * same result.  Returns 0 when launched, 1 for invalid arguments, 3 for a
    * CUDA error. */
