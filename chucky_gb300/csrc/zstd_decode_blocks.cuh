@@ -1433,8 +1433,10 @@ cudaError_t zd_launch(const ZWave& W, cudaStream_t st)
     return e;
   // Blocks per warp: one lane each when they share their tables, so more of
   // them cost no more instructions; but a sequence takes 250 cycles on its
-  // lane, so a few warps per scheduler are wanted first (12 per SM).
-  const uint64_t share = W.n * ((W.chunk_bytes >> 13) + 1) / (152 * 12);
+  // lane, so a few warps per scheduler are wanted first (12 per SM).  Blocks of
+  // 8 KiB are assumed, as this library's encoder makes them: stock frames of
+  // 128 KiB blocks are sixteen times fewer, and share no tables either.
+  const uint64_t share = W.n * ((W.chunk_bytes >> 13) + 1) / (uint64_t(device_sm_count()) * 12);
   uint32_t per = 1;
   while (per < 32 && per <= share)
     per *= 2;
