@@ -89,6 +89,8 @@ struct ZWave // one launch set's chunks and lists
 #define CHUCKY_ZSTD_SCRATCH (256ull << 20)
 #endif
 constexpr uint64_t kZdScratch = CHUCKY_ZSTD_SCRATCH;
+// chunks up to this size are decoded sequentially
+constexpr uint64_t kZdSequential = 64;
 // chunks whose frames' records are kept for one pass of the sequential decoder
 #ifndef CHUCKY_ZSTD_FRAMES
 #define CHUCKY_ZSTD_FRAMES (1ull << 20)

@@ -77,3 +77,9 @@ def test_launch_sets(decode_emu, chunk, per_set, n):
     groups = [min(10, n - g) for g in range(0, n, 10)]
     want = sum(5 * -(-g // per_set) + 1 for g in groups)
     assert run(decode_emu, chunk, n, 3 * chunk + n) == "ok %d\n" % want
+
+
+@pytest.mark.parametrize("chunk,launches", [(64, 1), (65, 6)])
+def test_tiny_chunks(decode_emu, chunk, launches):
+    """Chunks up to 64 bytes go to the sequential decoder at once."""
+    assert run(decode_emu, chunk, 8, chunk) == "ok %d\n" % launches
