@@ -23,6 +23,7 @@ struct TransposeArgs
   const uint64_t* row_off; // element offset of (row, 0) in the slot
   const uint64_t* col_off; // element offset of column x within a row
   int vector_ok;           // 16-byte runs stay contiguous and aligned
+  uint32_t run;            // elements per thread otherwise: 1 or 4
   uint32_t channels;       // 2..4: narrow innermost dim above a contiguous one
   uint64_t channel_off[4]; // (element offsets of the channels), 0: not so
 };

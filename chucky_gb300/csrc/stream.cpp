@@ -257,6 +257,15 @@ int Stream::setup_transpose()
   for (int d = 0; d < r && planar; ++d)
     planar = d == r - 3 || L.lifted_shape[d] == 1 ||
              (uint64_t(L.lifted_strides[d]) * P.bpe) % 16 == 0;
+  // Four elements per thread where they go to chunk rows of their own (every
+  // element another chunk; with a pair of rows per four, rows of some length,
+  // and for 8 bytes some more of them), and where the rows are long for u8
+  // (transpose_scalar_k has the figures).
+  const bool apart = cs == 1 && channels % 4 == 0;
+  const bool pairs = cs == 1 && channels % 2 == 0 && r >= 4 && L.lifted_shape[r - 3] >= 16 &&
+                     (P.bpe <= 4 || channels > 8);
+  const bool long_rows = P.bpe == 1 && L.lifted_strides[r - 1] == 1 && cs >= 64;
+  tr.run = apart || pairs || long_rows ? 4 : 1;
   if (planar) {
     tr.channels = uint32_t(channels);
     for (uint64_t c = 0; c < channels; ++c)

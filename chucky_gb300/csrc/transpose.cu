@@ -89,10 +89,17 @@ transpose_planar_k(TransposeArgs a, uint64_t ngroups)
 }
 
 // Elements one by one, where vectors do not stay whole: kRun consecutive ones
-// per thread, read with one or two vector loads and one division.  Bound by
-// its stores, an element each.
-constexpr uint32_t kRun = 4;
-template<typename T>
+// per thread (TransposeArgs::run), four read with one or two vector loads and
+// one division.  Bound by its stores, an element each: neighbouring threads
+// store side by side with one element each, four apart with four, which only
+// pays where the elements go to different chunk rows anyway.  us for 540 x 959
+// pixels x 4 frames, 1 and 4 per thread, u8 / u32, chunks of one channel and
+// 100 columns: 2 channels 14 and 12 / 9 and 10, 3: 20 and 22 / 12 and 11, 4: 24
+// and 18 / 16 and 15, 6: 39 and 33 / 44 and 36, 8: 57 and 36 / 59 and 39; 7
+// columns, 2 channels: 16 and 23 / 15 and 18.  Rows of u8 cut every 100
+// columns, 1080 x 2000 x 4 frames: 22 and 20; every 20: 22 and 29; every 5: 25
+// and 59.  u16 every 100: 22 and 24.
+template<typename T, uint32_t kRun>
 __global__ void __launch_bounds__(kThreads)
 transpose_scalar_k(TransposeArgs a, uint64_t first)
 {
@@ -128,6 +135,18 @@ int grid_for(uint64_t work)
   const uint64_t blocks = (work + kThreads - 1) / kThreads;
   const uint64_t cap = uint64_t(device_sm_count()) * 8;
   return int(blocks < cap ? (blocks ? blocks : 1) : cap);
+}
+
+template<typename T>
+cudaError_t launch_scalar(const TransposeArgs& a, uint64_t first, cudaStream_t st)
+{
+  const int g = grid_for((a.n - first + a.run - 1) / a.run);
+  if (a.run == 4)
+    transpose_scalar_k<T, 4><<<g, kThreads, 0, st>>>(a, first);
+  else
+    transpose_scalar_k<T, 1><<<g, kThreads, 0, st>>>(a, first);
+  note_launches(1);
+  return cudaGetLastError();
 }
 
 template<int kBpe>
@@ -180,21 +199,15 @@ cudaError_t launch_transpose(const TransposeArgs& a, cudaStream_t st)
     }
   }
   if (first < a.n) {
-    const int g = grid_for((a.n - first + kRun - 1) / kRun);
-    note_launches(1);
     switch (a.bpe) {
       case 1:
-        transpose_scalar_k<uint8_t><<<g, kThreads, 0, st>>>(a, first);
-        break;
+        return launch_scalar<uint8_t>(a, first, st);
       case 2:
-        transpose_scalar_k<uint16_t><<<g, kThreads, 0, st>>>(a, first);
-        break;
+        return launch_scalar<uint16_t>(a, first, st);
       case 4:
-        transpose_scalar_k<uint32_t><<<g, kThreads, 0, st>>>(a, first);
-        break;
+        return launch_scalar<uint32_t>(a, first, st);
       case 8:
-        transpose_scalar_k<uint64_t><<<g, kThreads, 0, st>>>(a, first);
-        break;
+        return launch_scalar<uint64_t>(a, first, st);
       default:
         return cudaErrorInvalidValue;
     }
