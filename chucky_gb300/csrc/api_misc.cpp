@@ -346,10 +346,12 @@ chucky_crc32c(const void* data, size_t len)
 namespace chucky {
 
 // `shared_encoder`: the stream encodes through a server's engine and holds
-// no encoder scratch of its own.
+// no encoder scratch of its own.  `device_slots`: with the device copies of the
+// delivery slots that a stream without a codec can do without.
 int estimate_stream(const tile_stream_configuration* config,
                     tile_stream_memory_info* info,
-                    bool shared_encoder)
+                    bool shared_encoder,
+                    bool device_slots)
 {
   if (!info)
     return 1;
@@ -378,7 +380,8 @@ int estimate_stream(const tile_stream_configuration* config,
                      (sa ? (nsh + 1) * sa : 0) + 64);
     // shard-order tables, scan scratch, both slots' offsets and sizes
     agg_dev += 4 * cap * M * 4 + (pos + 1) * 8 + 2 * ((pos + 1) * 8 + pos * 8 + 8);
-    if (chucky::delivery_through_device(*config, P)) // device copy of both slots
+    if (config->codec.id != CODEC_NONE ||
+        (device_slots && chucky::delivery_through_device(*config, P)))
       agg_dev += 2 * (cap * M * P.max_out + (sa ? (nsh + 1) * sa : 0) + 64);
     shard += V.shard_inner_count * V.cps_total * 16;
   }
@@ -430,7 +433,7 @@ extern "C" int
 tile_stream_gpu_memory_estimate(const tile_stream_configuration* config,
                                 tile_stream_memory_info* info)
 {
-  return chucky::estimate_stream(config, info, false);
+  return chucky::estimate_stream(config, info, false, true);
 }
 
 extern "C" int
@@ -445,7 +448,7 @@ tile_stream_gpu_advise_chunk_sizes(tile_stream_configuration* config,
   for (size_t t = target_chunk_bytes; t >= bpe; t >>= 1) {
     dims_budget_chunk_bytes(config->dimensions, config->rank, t, bpe, ratios);
     tile_stream_memory_info mem;
-    if (tile_stream_gpu_memory_estimate(config, &mem))
+    if (chucky::estimate_stream(config, &mem, false, false))
       return 1;
     if (mem.device_bytes <= budget_bytes)
       return 0;

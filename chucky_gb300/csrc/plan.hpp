@@ -94,14 +94,15 @@ uint64_t ravel(int rank,
                const int64_t* strides,
                uint64_t idx);
 
-// Whether a batch's shard-ordered bytes are gathered in device memory and
+// Whether a batch's shard-ordered bytes are best gathered in device memory and
 // moved to the host by the copy engine, rather than stored by the gather
 // kernel into mapped host memory.
 //
 // The copy engine moves 190 GB/s over the link, SM stores 94 GB/s, and the
 // next batch's kernels run beside the copy; but the copy is one more step
 // (about 8 us) behind the gather.  With a codec always (its tail kernel
-// needs the device copy); without one from kDeviceSlotBytes per batch on.
+// needs the device copy); without one from kDeviceSlotBytes per batch on, where
+// there is room for the copies (Stream::setup_device_slots).
 constexpr uint64_t kDeviceSlotBytes = 1ull << 20;
 inline bool delivery_through_device(const tile_stream_configuration& cfg, const StreamPlan& P)
 {

@@ -24,10 +24,12 @@
 namespace chucky {
 tile_stream_gpu* create_stream(const tile_stream_configuration* config,
                                shard_sink* sink,
-                               Engine* engine);
+                               Engine* engine,
+                               bool device_slots);
 int estimate_stream(const tile_stream_configuration* config,
                     tile_stream_memory_info* info,
-                    bool shared_encoder);
+                    bool shared_encoder,
+                    bool device_slots);
 } // namespace chucky
 
 namespace {
@@ -71,6 +73,14 @@ double now_s()
   return duration<double>(steady_clock::now().time_since_epoch()).count();
 }
 
+// What a configuration's stream is charged, and whether it gets the device
+// copies of its delivery slots.
+struct Need
+{
+  uint64_t bytes = 0;
+  bool device_slots = false;
+};
+
 struct Idle
 {
   tile_stream_gpu* s;
@@ -88,7 +98,7 @@ struct chucky_server
   std::mutex m;
   std::condition_variable cv;
   std::list<Idle> idle; // least recently released first
-  std::map<std::string, uint64_t> need; // device estimate per configuration
+  std::map<std::string, Need> need; // per configuration
   uint64_t resident = 0;
   int open = 0;
   // statistics
@@ -96,6 +106,34 @@ struct chucky_server
   uint64_t requests = 0, input_bytes = 0, created = 0, reused = 0, evicted = 0;
   uint64_t peak_resident = 0, peak_open = 0;
 };
+
+namespace {
+
+// Planning a configuration costs host time: once per key.  The copies that a
+// stream without a codec can do without are for it where as many such streams
+// as the server opens fit the budget, so that they keep no request out.
+bool need_of(chucky_server* s, const tile_stream_configuration* c, const std::string& key, Need& n)
+{
+  {
+    std::lock_guard<std::mutex> lk(s->m);
+    auto it = s->need.find(key);
+    if (it != s->need.end()) {
+      n = it->second;
+      return true;
+    }
+  }
+  tile_stream_memory_info least{}, full{};
+  if (chucky::estimate_stream(c, &least, s->engine != nullptr, false) ||
+      chucky::estimate_stream(c, &full, s->engine != nullptr, true))
+    return false;
+  n.device_slots = full.device_bytes <= s->cfg.hbm_budget_bytes / uint64_t(s->cfg.max_streams);
+  n.bytes = n.device_slots ? full.device_bytes : least.device_bytes;
+  std::lock_guard<std::mutex> lk(s->m);
+  s->need[key] = n;
+  return true;
+}
+
+} // namespace
 
 struct chucky_request
 {
@@ -158,21 +196,10 @@ chucky_server_open(chucky_server* s,
   if (cudaSetDevice(s->device) != cudaSuccess)
     return nullptr;
   const std::string key = config_key(config);
-  uint64_t need = 0;
-  {
-    std::lock_guard<std::mutex> lk(s->m);
-    auto it = s->need.find(key);
-    if (it != s->need.end())
-      need = it->second;
-  }
-  if (!need) { // planning a configuration costs host time: once per key
-    tile_stream_memory_info info{};
-    if (chucky::estimate_stream(config, &info, s->engine != nullptr))
-      return nullptr;
-    need = info.device_bytes;
-    std::lock_guard<std::mutex> lk(s->m);
-    s->need[key] = need;
-  }
+  Need n;
+  if (!need_of(s, config, key, n))
+    return nullptr;
+  const uint64_t need = n.bytes;
   if (need > s->cfg.hbm_budget_bytes)
     return nullptr;
   const auto deadline = std::chrono::steady_clock::now() +
@@ -222,7 +249,8 @@ chucky_server_open(chucky_server* s,
         lk.unlock();
         for (Idle& v : victims)
           tile_stream_gpu_destroy(v.s);
-        tile_stream_gpu* st = chucky::create_stream(config, sink, s->engine.get());
+        tile_stream_gpu* st =
+          chucky::create_stream(config, sink, s->engine.get(), n.device_slots);
         if (!st) {
           lk.lock();
           s->resident -= need;
@@ -263,28 +291,18 @@ chucky_server_prewarm(chucky_server* s,
     if (!c)
       continue;
     const std::string key = config_key(c);
-    uint64_t need = 0;
-    {
-      std::lock_guard<std::mutex> lk(s->m);
-      auto it = s->need.find(key);
-      if (it != s->need.end())
-        need = it->second;
-    }
-    if (!need) {
-      tile_stream_memory_info info{};
-      if (chucky::estimate_stream(c, &info, s->engine != nullptr))
-        continue;
-      need = info.device_bytes;
-      std::lock_guard<std::mutex> lk(s->m);
-      s->need[key] = need;
-    }
+    Need what;
+    if (!need_of(s, c, key, what))
+      continue;
+    const uint64_t need = what.bytes;
     {
       std::lock_guard<std::mutex> lk(s->m);
       if (s->resident + need > s->cfg.hbm_budget_bytes)
         continue;
       s->resident += need;
     }
-    tile_stream_gpu* st = chucky::create_stream(c, sink, s->engine.get());
+    tile_stream_gpu* st =
+      chucky::create_stream(c, sink, s->engine.get(), what.device_slots);
     std::lock_guard<std::mutex> lk(s->m);
     if (!st) {
       s->resident -= need;

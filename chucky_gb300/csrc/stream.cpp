@@ -471,7 +471,6 @@ void Stream::build_luts(int l,
 int Stream::setup_aggregate()
 {
   uint64_t max_positions = 0;
-  slots_on_device = delivery_through_device(cfg, P);
   for (int l = 0; l < P.nlod; ++l) {
     const LevelPlan& V = P.lv[l];
     const uint32_t slots = std::max<uint32_t>(V.batch_active, 1);
@@ -510,8 +509,6 @@ int Stream::setup_aggregate()
       CK(cudaMalloc(&D.d_offsets, 2 * (positions + 1) * 8));
       D.real_sizes = D.d_offsets + positions + 1;
       CK(cudaHostAlloc(&D.data, data, cudaHostAllocMapped));
-      if (slots_on_device)
-        CK(cudaMalloc(&D.d_data, data));
     }
     // shard state (src/zarr/shard_delivery.c:10-34); the index lives on
     // the device
@@ -546,6 +543,45 @@ int Stream::setup_aggregate()
   }
   agg_scratch_slot = (max_positions + 1) * size_t(P.nlod);
   CK(cudaMalloc(&d_agg_scratch, 2 * agg_scratch_slot * 8));
+  return setup_device_slots();
+}
+
+// The delivery slots' device copies, behind everything else that the stream
+// needs.  A stream without a codec does without them (its gather stores into
+// the mapped slots) where its server has no room for them in the budget, where
+// they would take more than an eighth of the device's free memory, and where
+// they cannot be had.
+int Stream::setup_device_slots()
+{
+  slots_on_device = delivery_through_device(cfg, P);
+  const bool needed = cfg.codec.id != CODEC_NONE;
+  if (slots_on_device && !needed) {
+    uint64_t bytes = 0;
+    size_t room = 0, all = 0;
+    for (const DeliverySlot& S : slot)
+      for (int l = 0; l < P.nlod; ++l)
+        bytes += S.lv[l].data_cap;
+    slots_on_device =
+      device_slots_allowed && cudaMemGetInfo(&room, &all) == cudaSuccess && bytes <= room / 8;
+  }
+  if (!slots_on_device)
+    return 0;
+  for (DeliverySlot& S : slot)
+    for (int l = 0; l < P.nlod; ++l) {
+      const cudaError_t e = cudaMalloc(&S.lv[l].d_data, S.lv[l].data_cap);
+      if (e == cudaSuccess)
+        continue;
+      if (needed)
+        CK(e);
+      cudaGetLastError();
+      for (DeliverySlot& T : slot)
+        for (int k = 0; k < P.nlod; ++k) {
+          cudaFree(T.lv[k].d_data);
+          T.lv[k].d_data = nullptr;
+        }
+      slots_on_device = false;
+      return 0;
+    }
   return 0;
 }
 
@@ -1526,7 +1562,8 @@ namespace chucky {
 
 tile_stream_gpu* create_stream(const tile_stream_configuration* config,
                                shard_sink* sink,
-                               Engine* engine)
+                               Engine* engine,
+                               bool device_slots)
 {
   if (!config || !sink || !sink->open)
     return nullptr;
@@ -1536,6 +1573,7 @@ tile_stream_gpu* create_stream(const tile_stream_configuration* config,
   s->w.append = vt_append;
   s->w.flush = vt_flush;
   s->impl.engine = engine;
+  s->impl.device_slots_allowed = device_slots;
   if (s->impl.init(config, sink)) {
     s->impl.release();
     delete s;
@@ -1550,7 +1588,7 @@ extern "C" tile_stream_gpu*
 tile_stream_gpu_create(const tile_stream_configuration* config,
                        shard_sink* sink)
 {
-  return chucky::create_stream(config, sink, nullptr);
+  return chucky::create_stream(config, sink, nullptr, true);
 }
 
 extern "C" writer_result

@@ -164,6 +164,7 @@ struct Stream
   uint64_t agg_scratch_slot = 0; // entries per delivery slot
   DeliverySlot slot[2];
   bool slots_on_device = false; // batches are gathered on the device first
+  bool device_slots_allowed = true;
   cudaEvent_t ev_batch[2] = {};
   int next_slot = 0;
   uint64_t batch_seq = 0;
@@ -211,6 +212,7 @@ struct Stream
   int setup_transpose();
   int setup_lod();
   int setup_aggregate();
+  int setup_device_slots();
   void build_luts(int l,
                   uint32_t n_active,
                   const uint32_t* eps,

@@ -9,7 +9,9 @@
  *
  *   * admission: a request is admitted once fewer than `max_streams`
  *     requests are open and its stream fits the HBM budget (the sum of the
- *     device-memory estimates of the resident streams).  A finished
+ *     device-memory estimates of the resident streams; a stream without a
+ *     codec gets device copies of its delivery slots only where max_streams
+ *     such streams fit with them).  A finished
  *     request's stream stays resident, idle, and is restarted for the next
  *     request with the same configuration (no allocation); idle streams of
  *     other configurations are released when room is needed;

@@ -60,13 +60,17 @@ extern "C"
   struct tile_stream_gpu;
 
   /* Device/host memory a stream with this config would hold; nothing is
-   * allocated.  0 on success.  Replaces src/stream.gpu.h:41-43. */
+   * allocated.  0 on success.  Replaces src/stream.gpu.h:41-43.  A stream
+   * without a codec whose batches are 1 MiB or more holds device copies of its
+   * delivery slots; they are counted here, but it does without them where they
+   * would take more than an eighth of the device's free memory. */
   int tile_stream_gpu_memory_estimate(
     const struct tile_stream_configuration* config,
     struct tile_stream_memory_info* info);
 
   /* Largest power-of-two chunk (from target_chunk_bytes down) whose memory
-   * estimate fits budget_bytes; edits config->dimensions.  0 on success.
+   * estimate fits budget_bytes (the copies that a stream can do without, as
+   * above, aside); edits config->dimensions.  0 on success.
    * Replaces src/stream.gpu.h:45-52. */
   int tile_stream_gpu_advise_chunk_sizes(
     struct tile_stream_configuration* config,
