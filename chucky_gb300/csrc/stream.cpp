@@ -1037,10 +1037,14 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
     // The copies run on the slot's encoder stream, beside the index kernel
     // and the next batch's layout and gather (or, without a codec, its
     // epochs): nothing else is queued there until the batch is delivered.
-    // A stream of a server keeps to its aggregation stream: many streams
-    // share the device's hardware queues, and one more of them in use was
-    // not faster there.
-    const bool apart = !engine;
+    // A server's stream with a codec keeps to its aggregation stream: many
+    // streams share the device's hardware queues, and one more of them in use
+    // was not faster there.  Without a codec that would be the compute stream,
+    // and the next epoch would wait for the link (the four arrays of a mixed
+    // server pass, uncompressed: the first alone 0.67 ms in line, 0.50 apart,
+    // two 5.72 and 5.22, all 8.39 and 8.33; stored by the gather 0.58, 5.57,
+    // 9.16).
+    const bool apart = !engine || !coded;
     const cudaStream_t sx = apart ? s_agg : sa;
     if (apart) {
       so = se;
