@@ -1029,7 +1029,7 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
     return 1;
   CK(launch_aggregate(ab, d_agg_scratch + si * agg_scratch_slot,
                       slots_on_device ? nullptr : &ib, sa));
-  if (timed_end(sa))
+  if (!slots_on_device && timed_end(sa))
     return 1;
   CK(cudaEventRecord(ev_agg_done[si], sa)); // the compressed slots are free
   cudaStream_t so = sa;
@@ -1053,6 +1053,8 @@ int Stream::kick_batch(uint32_t n_epochs, const uint32_t* epoch_masks)
         CK(cudaStreamWaitEvent(sx, ev_agg_done[si], 0));
     }
     CK(launch_index(ib, sx));
+    if (timed_end(sx)) // (the aggregation's timer: layout, gather and index)
+      return 1;
     if (apart)
       CK(cudaEventRecord(ev_index_done[si], sx));
     if (copy_out(S, so))
