@@ -79,7 +79,10 @@ __global__ void __launch_bounds__(kThreads) reduce_k(T* values, ReduceLevel L, i
 }
 
 // The pyramid's top, levels of at most kTailElems elements, in one CTA: a
-// launch each cost 4 to 6 us for work of a few hundred windows.
+// launch each cost 4 to 6 us for work of a few hundred windows.  All levels of
+// the i16 volume of 16 x 200 x 328 reduced, by kTailElems: 22.2 us with 0 (a
+// launch each), 20.2 with 1024, 19.9 with 4096, 20.3 with 16384, 33.6 with 65536;
+// of 32 x 400 x 656: 39.7, 33.5, 33.8, 33.8, 52.3.
 constexpr uint64_t kTailElems = 4096;
 constexpr int kTailThreads = 1024, kTailLevels = 16;
 struct ReduceTail

@@ -98,11 +98,14 @@ uint64_t ravel(int rank,
 // moved to the host by the copy engine, rather than stored by the gather
 // kernel into mapped host memory.
 //
-// The copy engine moves 190 GB/s over the link, SM stores 94 GB/s, and the
-// next batch's kernels run beside the copy; but the copy is one more step
-// (about 8 us) behind the gather.  With a codec always (its tail kernel
-// needs the device copy); without one from kDeviceSlotBytes per batch on, where
-// there is room for the copies (Stream::setup_device_slots).
+// The copy engine moves 191 GB/s over the link, beside the next batch's kernels;
+// the gather stores 67 MB at 147 GB/s (chunks of 32 KiB) to 178 (of 8 MiB), and
+// the compute stream waits for it.  But the copy is one more step behind a
+// gather on the device: a pass of a single batch of 4 MiB chunks takes 1,165 us
+// with it and 1,152 without, one of two RGB batches 511 and 695.  With a codec
+// always (its tail kernel needs the device copy); without one from
+// kDeviceSlotBytes per batch on, where there is room for the copies
+// (Stream::setup_device_slots).
 constexpr uint64_t kDeviceSlotBytes = 1ull << 20;
 inline bool delivery_through_device(const tile_stream_configuration& cfg, const StreamPlan& P)
 {
