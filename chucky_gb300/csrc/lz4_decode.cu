@@ -661,8 +661,6 @@ lz4_decode_k(const uint8_t* in,
 {
   CHUCKY_DYN_SHARED(uint4, sm);
   LzShared<NT>& S = *reinterpret_cast<LzShared<NT>*>(sm);
-  __shared__ uint64_t left_ip[NT / 32], left_op[NT / 32];
-  __shared__ uint32_t left[NT / 32];
   auto block = [&](uint64_t c, uint64_t ip, uint64_t op) {
     const uint8_t* src = in + in_off[c];
     const uint64_t n = in_size[c];
