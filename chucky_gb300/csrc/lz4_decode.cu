@@ -128,11 +128,24 @@ __device__ __forceinline__ uint32_t lz4_decode_warp(const uint8_t* src,
       return kDecodeTruncated;
     if (lit > chunk_bytes - to)
       return kDecodeOverrun;
-    if (kVec && lit >= 256)
-      warp_copy(dst + to, src + at, lit);
-    else
+    if (!kVec) {
       for (uint64_t j = lane; j < lit; j += 32)
         dst[to + j] = src[at + j];
+    } else if (lit >= 256) {
+      warp_copy(dst + to, src + at, lit);
+    } else { // four loads in flight: one by one they took a tenth longer
+      for (uint32_t j = lane; j < uint32_t(lit); j += 128) {
+        uint8_t v[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u)
+          if (j + 32 * u < lit)
+            v[u] = src[at + j + 32 * u];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u)
+          if (j + 32 * u < lit)
+            dst[to + j + 32 * u] = v[u];
+      }
+    }
     at += lit;
     to += lit;
     if (at == n) // the last sequence has literals only
@@ -446,11 +459,13 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
       // behind a few literals (constant data is one after another) are known
       // by their length bytes: no window is parsed for them
       peek = false;
-      const uint32_t t = src[ip], lit = t >> 4;
-      const bool run = lit == 15;
-      const uint64_t at = ip + 1 + (run ? 0 : lit + 2) + lane;
-      const bool full = lane >= lz4_peek_bytes<NT>(chunk_bytes) || (at < n && src[at] == 255);
-      if (__all_sync(kAll, full && (run || (t & 15) == 15))) {
+      const uint32_t bytes = lz4_peek_bytes<NT>(chunk_bytes);
+      auto full = [&](uint64_t at) { return lane >= bytes || (at + lane < n && src[at + lane] == 255); };
+      bool is_long = full(ip + 1); // (loaded beside the token, not behind it)
+      const uint32_t t = src[ip];
+      if (t >> 4 != 15)
+        is_long = (t & 15) == 15 && full(ip + 3 + (t >> 4));
+      if (__all_sync(kAll, is_long)) {
         bool last = false;
         if (!run_long(last))
           return false;
@@ -625,19 +640,22 @@ __device__ bool lz4_decode_tiles(LzShared<NT>& S,
 
 // Whether a block has few sequences, by its size: it saved less than a 64th of
 // its bytes (matches are rare), or takes less than an eighth (a sequence is
-// three bytes or more).  Not one that starts with kLongSequence literals, which
-// a CTA copies sooner.
-__device__ __forceinline__ bool lz4_few_sequences(const uint8_t* src, uint64_t n, uint64_t chunk_bytes)
+// three bytes or more).
+__device__ __forceinline__ bool lz4_few_by_size(uint64_t n, uint64_t chunk_bytes)
 {
-  if (n < chunk_bytes - chunk_bytes / 64)
-    return n < chunk_bytes / 8;
+  return n < chunk_bytes / 8 || n >= chunk_bytes - chunk_bytes / 64;
+}
+
+// Whether it starts with kLongSequence literals, which a CTA copies sooner
+// (every lane of a warp).
+__device__ __forceinline__ bool lz4_long_start(const uint8_t* src, uint64_t n)
+{
   constexpr uint32_t kBytes = kLongSequence / 255 + 1;
   static_assert(kBytes > 32 && kBytes <= 96, "two or three length bytes per lane");
-  const uint32_t lane = threadIdx.x & 31;
   bool full = n > kBytes && src[0] >> 4 == 15;
-  for (uint32_t k = lane; k < kBytes && full; k += 32)
+  for (uint32_t k = threadIdx.x & 31; k < kBytes && full; k += 32)
     full = src[1 + k] == 255;
-  return !__all_sync(0xffffffffu, full);
+  return __all_sync(0xffffffffu, full);
 }
 
 // kMany: CTAs below `groups` take `per` blocks each (a warp a block at most): the
@@ -671,7 +689,9 @@ lz4_decode_k(const uint8_t* in,
     if (threadIdx.x < 32) {
       uint64_t ip0 = 0, op0 = 0;
       const uint32_t st =
-        ok ? uint32_t(kDecodeOk) : lz4_decode_serial(src, n, dst, chunk_bytes, 0, ip0, op0);
+        ok      ? uint32_t(kDecodeOk)
+        : kMany ? lz4_decode_serial(src, n, dst, chunk_bytes, 0, ip0, op0)
+                : lz4_decode_warp<false>(src, n, dst, chunk_bytes, 0, ip0, op0);
       if (threadIdx.x == 0)
         status[c] = st;
     }
@@ -682,29 +702,36 @@ lz4_decode_k(const uint8_t* in,
     __shared__ uint32_t left[NT / 32];
     const uint32_t warp = threadIdx.x >> 5;
     const bool group = blockIdx.x < groups;
-    const uint64_t c0 = group ? uint64_t(blockIdx.x) * per : uint64_t(blockIdx.x - groups);
-    const uint32_t m = !group ? 1 : uint32_t(n_chunks - c0 < per ? n_chunks - c0 : per);
-    if (warp < m) {
-      const uint64_t c = c0 + warp, n = in_size[c];
-      const uint8_t* src = in + in_off[c];
-      const bool few = lz4_few_sequences(src, n, chunk_bytes);
-      uint64_t ip = 0, op = 0;
-      uint32_t st = group == few ? kDecodeLeft : kDecodeOk; // (Ok: another CTA's block)
-      if (group && few) {
-        st = lz4_decode_serial(src, n, out + c * out_stride, chunk_bytes, worth, ip, op);
-        if (st != kDecodeLeft && (threadIdx.x & 31) == 0)
-          status[c] = st;
+    uint64_t c0 = blockIdx.x - groups;
+    uint32_t m = 1;
+    if (group) {
+      c0 = uint64_t(blockIdx.x) * per;
+      m = uint32_t(n_chunks - c0 < per ? n_chunks - c0 : per);
+      if (warp < m) {
+        const uint64_t c = c0 + warp, n = in_size[c];
+        const uint8_t* src = in + in_off[c];
+        uint64_t ip = 0, op = 0;
+        uint32_t st = kDecodeOk; // (another CTA's block)
+        if (lz4_few_by_size(n, chunk_bytes) && !lz4_long_start(src, n)) {
+          st = lz4_decode_serial(src, n, out + c * out_stride, chunk_bytes, worth, ip, op);
+          if (st != kDecodeLeft && (threadIdx.x & 31) == 0)
+            status[c] = st;
+        }
+        if ((threadIdx.x & 31) == 0) {
+          left_ip[warp] = ip;
+          left_op[warp] = op;
+          left[warp] = st;
+        }
       }
-      if ((threadIdx.x & 31) == 0) {
-        left_ip[warp] = ip;
-        left_op[warp] = op;
-        left[warp] = st;
-      }
+      __syncthreads();
+    } else if (const uint64_t n = in_size[c0]; lz4_few_by_size(n, chunk_bytes)) {
+      const bool keep = warp == 0 && lz4_long_start(in + in_off[c0], n);
+      if (!__syncthreads_or(keep))
+        return; // (a warp's block)
     }
-    __syncthreads();
     for (uint32_t k = 0; k < m; ++k)
-      if (left[k] == kDecodeLeft) // (the whole CTA)
-        block(c0 + k, left_ip[k], left_op[k]);
+      if (!group || left[k] == kDecodeLeft) // (the whole CTA)
+        block(c0 + k, group ? left_ip[k] : 0, group ? left_op[k] : 0);
   } else {
     for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x)
       block(c, 0, 0);
@@ -818,7 +845,7 @@ lz4_decode_pair_k(const uint8_t* in,
         uint64_t ip = 0, op = 0;
         const uint32_t st =
           ok ? uint32_t(kDecodeOk)
-             : lz4_decode_serial(src, n, dst, chunk_bytes, 0, ip, op);
+             : lz4_decode_warp<false>(src, n, dst, chunk_bytes, 0, ip, op);
         if (threadIdx.x == 0)
           status[c] = st;
       }
@@ -930,10 +957,10 @@ cudaError_t launch_lz4_decode(const uint8_t* in,
   // warps on an SM, against the CTA's 4.7 us per KiB of each of its chunks.
   // us, every chunk to a CTA / so / every chunk to a warp:
   //   chunks x bytes     sensor counts   volume           constant or random
-  //   1,467 x 4,440       80  82  260     72  38  41      76  18  33
-  //   4,096 x 4,096      127 132  325    149  44  41     141  23  36
-  //   4,096 x 8,192      279 288  715    251  86  84     204  29  64
-  //   2,048 x 16,384     288 294 1114    247 144 146     199  37  95
+  //   1,467 x 4,440       80  81  260     72  32  38      76  16  30
+  //   4,096 x 4,096      126 130  325    149  38  40     141  20  34
+  //   4,096 x 8,192      280 287  719    251  82  81     204  26  62
+  //   2,048 x 16,384     288 293 1111    247 129 143     199  36  93
   // Chunks of up to 512 bytes are all left to single warps (608 of 256 bytes: 3.3
   // us on the device, 9.2 with CTAs; 64 sensor ones of 500 bytes 13.5 and 10.6),
   // and so are many of up to 1 KiB (4,096 of sensor counts: 54 and 82 us).
